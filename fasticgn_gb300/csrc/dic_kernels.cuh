@@ -11,6 +11,7 @@
 #pragma once
 
 #include <climits>
+#include <cstddef>
 #include <cstdint>
 #include <cuda.h>            // CUtensorMap (the type only; maps are encoded through the runtime's driver entry point)
 #include <cuda_runtime.h>
@@ -1010,6 +1011,16 @@ __host__ __device__ constexpr int px_pitch(int w) { return (w + 3) & ~3; }
 // (fma.rn.f32x2, sm_100 and later) round each half like the scalar operation, so the
 // values are the scalar Horner forms' bit for bit, in half the instructions.
 __device__ __forceinline__ float2 k2(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 csub(float2 a, float2 b)
+{
+  unsigned long long ra, rb, rd;
+  memcpy(&ra, &a, 8);
+  memcpy(&rb, &b, 8);
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(rd) : "l"(ra), "l"(rb));
+  float2 d;
+  memcpy(&d, &rd, 8);
+  return d;
+}
 __device__ __forceinline__ void bspline_weights2(float2 d, float2 (&w)[4])
 {
   w[0] = __fmul2_rn(__ffma2_rn(__ffma2_rn(k2(-144.0f / 336.0f), d, k2(342.0f / 336.0f)), d, k2(-198.0f / 336.0f)), d);
@@ -1072,16 +1083,6 @@ __device__ __forceinline__ float sample_pixels(const PixelTile& T, const float* 
   }
   const float* g = tar + ((size_t)(iy - 1) * pitch + (ix - 1));   // images < 2^31 pixels
   return eval_pixels(wt, [&](int n, int m) { return __ldg(g + (size_t)n * pitch + m); });
-}
-
-// A sample whose support lies in the window (the caller has checked): no tests.
-__device__ __forceinline__ float sample_window(const PixelTile& T, int row, float gxp, float gyp)
-{
-  float2 wt[4];
-  int ix, iy;
-  pixel_setup(gxp, gyp, wt, ix, iy);
-  const int a = T.s + ((iy - 1 - T.oy) * T.bx + (ix - 1 - T.ox));
-  return eval_pixels(wt, [&](int n, int m) { return px_smem[a + n * row + m]; });
 }
 
 // Column walk under pixel sampling: whether every sample of the current warp lies in the
@@ -1165,8 +1166,186 @@ __device__ __forceinline__ ColumnSums px_column_checked(const float* __restrict_
   return c;
 }
 
+// Adds one sample (target value t, reference texel v = {ref, gx, gy, 0}) to the nine sums.
+// __fmul_rn / __fadd_rn: never contracted, so these match k_poi_prepare's G bit for bit.
+__device__ __forceinline__ void add_sample(ColumnSums& c, float t, const float4& v, float t0, float fly)
+{
+  const float tau = t - t0;
+  const float rc = v.x - t0;
+  c.A0 += tau;
+  c.A1 = fmaf(tau, tau, c.A1);
+  c.A2 = fmaf(tau, rc, c.A2);
+  const float gt = __fmul_rn(v.y, tau), ht = __fmul_rn(v.z, tau);
+  c.B0 = __fadd_rn(c.B0, gt);
+  c.B2 = fmaf(gt, fly, c.B2);
+  c.B3 = __fadd_rn(c.B3, ht);
+  c.B5 = fmaf(ht, fly, c.B5);
+}
+
+// floor of both halves for 0 <= g < 2^23: t = g + 2^23 rounded down holds the integer in its
+// low mantissa bits (0x4B000000 + floor) and t - 2^23 is the floor as a float, exactly.  Two
+// packed additions, against a rounding and a conversion per axis on the quarter-rate unit.
+constexpr unsigned kFloorBias = 0x4B000000u;
+constexpr float kFloorMagic = 8388608.0f;
+__device__ __forceinline__ float2 floor_bits2(float2 g)
+{
+  unsigned long long rg, rb, rd;
+  const float2 b = k2(kFloorMagic);
+  memcpy(&rg, &g, 8);
+  memcpy(&rb, &b, 8);
+  asm("add.rm.f32x2 %0, %1, %2;" : "=l"(rd) : "l"(rg), "l"(rb));
+  float2 d;
+  memcpy(&d, &rd, 8);
+  return d;
+}
+
+// A float of the window at a byte address of the shared space, as one load with an immediate
+// offset.  Not volatile, so the compiler may move it: its address comes from px_base, which is
+// pinned after the wait for the window's copy.
+template <int kOff>
+__device__ __forceinline__ float px_at(unsigned byte)
+{
+  float v;
+  asm("ld.shared.f32 %0, [%1+%2];" : "=f"(v) : "r"(byte), "n"(kOff));
+  return v;
+}
+__device__ __forceinline__ unsigned px_base()
+{
+  unsigned b = (unsigned)__cvta_generic_to_shared(px_smem);
+  asm volatile("" : "+r"(b)::"memory");
+  return b;
+}
+
+// The rows of one subset column whose samples all lie in the range and have their support in
+// the window (window_covers): the lane's nine sums, rows in order.  A row's 4 x 4 support
+// overlaps the one of the row before it in three rows of pixels, as long as both start in the
+// same column one row apart: those twelve pixels stay in registers (q, whose rows rotate by
+// unrolling) and a row loads four.  Where a lane's support steps otherwise (its warped column
+// or row crosses a pixel boundary) the warp reloads the other twelve (a third of the rows at
+// 1 % strain).  The rows go in groups of four without tests inside; a subset has an odd number
+// of rows, so the last group has three or one.  `mask`: the calling lanes.
+//
+// What bounds it: issue slots (98 instructions a row before, 86 now, of which 24 are the weights'
+// twelve packed products, two slots of the FMA pipe each) and the reference texel's trip to L2.
+// 96 registers hold a whole group in flight, so 20 resident warps do better than the 32 that
+// 64 registers allowed (2.86 against 3.18 ms of IC-GN on a 2048x2048 pair, 254 016 POIs, with
+// the lattice loop below; 24 warps 2.85, 16 warps 3.1).  Prefetching the texel a row ahead,
+// scalar weights and a packed form of add_sample moved the time by 1 % or less either way.
+struct ColumnRows
+{
+  float q[4][4];
+  const float4* rp;
+  float2 pxy, axy, Wy, fly;
+  unsigned org, pitch, expect, mask;
+  float t0;
+  int w;
+};
+template <int kN>
+__device__ __forceinline__ void px_row_group(ColumnRows& S, ColumnSums& c)
+{
+#pragma unroll
+  for (int k = 0; k < kN; ++k)
+  {
+    const float4 cur = __ldg(S.rp);
+    S.rp += S.w;
+    const float2 g = __fadd2_rn(S.pxy, __ffma2_rn(S.Wy, S.fly, S.axy));
+    const float2 bits = floor_bits2(g);
+    const float2 d = csub(g, __fadd2_rn(bits, k2(-kFloorMagic)));
+    const unsigned a = S.org + 4u * __float_as_uint(bits.x) + S.pitch * __float_as_uint(bits.y);
+    const unsigned last = a + 3 * S.pitch;
+    if (!__all_sync(S.mask, a == S.expect))
+    {
+      // keeps this a branch: as predicated loads the twelve cost their issue slots every row
+      asm volatile("bar.warp.sync %0;" ::"r"(S.mask));
+#pragma unroll
+      for (int n = 0; n < 3; ++n)
+      {
+        const unsigned b = a + n * S.pitch;
+        S.q[(n + k) & 3][0] = px_at<0>(b);
+        S.q[(n + k) & 3][1] = px_at<4>(b);
+        S.q[(n + k) & 3][2] = px_at<8>(b);
+        S.q[(n + k) & 3][3] = px_at<12>(b);
+      }
+    }
+    S.q[(3 + k) & 3][0] = px_at<0>(last);
+    S.q[(3 + k) & 3][1] = px_at<4>(last);
+    S.q[(3 + k) & 3][2] = px_at<8>(last);
+    S.q[(3 + k) & 3][3] = px_at<12>(last);
+    S.expect = a + S.pitch;
+    float2 wt[4];
+    bspline_weights2(d, wt);
+    const float t = eval_pixels(wt, [&](int n, int m) { return S.q[(n + k) & 3][m]; });
+    add_sample(c, t, cur, S.t0, S.fly.x);
+    S.fly = __fadd2_rn(S.fly, k2(1.f));
+  }
+}
+__device__ __forceinline__ void px_column_rows(ColumnSums& c, const PixelTile& T, const float4* __restrict__ rp, int w,
+                                               float2 pxy, float2 axy, float2 Wy, float t0, int ry, unsigned mask)
+{
+  ColumnRows S;
+  S.pitch = 4u * (unsigned)T.bx;
+  // byte address of the support's first pixel: org + 4 * bits(x) + pitch * bits(y)
+  S.org = px_base() + 4u * (unsigned)T.s - (S.pitch * (unsigned)(T.oy + 1) + 4u * (unsigned)(T.ox + 1)) -
+          kFloorBias * (S.pitch + 4u);
+  S.expect = 1u;   // no address: the first row loads its whole support
+  S.mask = mask;
+  S.pxy = pxy;
+  S.axy = axy;
+  S.Wy = Wy;
+  S.fly = k2((float)-ry);
+  S.t0 = t0;
+  S.w = w;
+  S.rp = rp;
+#pragma unroll 1
+  for (int r = (2 * ry + 1) >> 2; r > 0; --r) px_row_group<4>(S, c);
+  if (ry & 1)
+    px_row_group<3>(S, c);
+  else
+    px_row_group<1>(S, c);
+}
+
+// The same for an iteration on the pixel lattice (on_lattice: the first one from an FFTCC
+// seed): a sample is the pixel itself.  src: the column's first sample in px_smem.  Against the
+// checked loop, which it ran before, 1.13 -> 0.58 ms for the first iteration of the 2048x2048
+// pair.  Not inlined: its registers beside the row loop's slowed every other iteration by 15 %.
+__device__ __noinline__ ColumnSums px_column_lattice(int src, int pitch, const float4* __restrict__ rp, int w, float t0,
+                                                     int ry)
+{
+  ColumnSums c{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
+  const float* p = px_smem + src;
+  float fly = (float)-ry;
+#pragma unroll 4
+  for (int r = 0; r < 2 * ry + 1; ++r)
+  {
+    add_sample(c, *p, __ldg(rp), t0, fly);
+    p += pitch;
+    rp += w;
+    fly += 1.f;
+  }
+  return c;
+}
+
+// One column's sums of an iteration: lane column flx under warp W, in the form the iteration
+// allows (covered: window_covers, lat: on_lattice, both warp-uniform).
+__device__ __forceinline__ ColumnSums px_column(const PixelTile& T, const float* __restrict__ tar,
+                                                const float4* __restrict__ ref_col, int w, int h, float px, float py,
+                                                const float (&W)[6], float flx, float t0, int ry, bool covered, bool lat,
+                                                unsigned mask)
+{
+  ColumnSums c{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
+  const float ax = fmaf(W[0], flx, W[2]), ay = fmaf(W[3], flx, W[5]);
+  if (!covered)
+    c = px_column_checked(tar, w, h, T, ref_col, px, py, W[0], W[1], W[2], W[3], W[4], W[5], flx, t0, ry, lat ? 1 : 0);
+  else if (lat)
+    c = px_column_lattice(T.s + ((int)(py + fmaf(W[4], (float)-ry, ay)) - T.oy) * T.bx + ((int)(px + ax) - T.ox), T.bx,
+                          ref_col, w, t0, ry);
+  else
+    px_column_rows(c, T, ref_col, w, make_float2(px, py), make_float2(ax, ay), make_float2(W[1], W[4]), t0, ry, mask);
+  return c;
+}
+
 // Sample sources of icgn_solve: the global coefficient table, a coefficient block staged
-// in shared memory (k_icgn_tile), or the target pixels (k_icgn_px).
+// in shared memory (k_icgn_tile); of icgn_solve_pair also the target pixels (k_icgn_pair_px).
 constexpr int kSrcTable = 0, kSrcCoefTile = 1, kSrcPixels = 2;
 
 // Rows of the column walk unrolled together (their gathers in flight at once), and the
@@ -1228,62 +1407,10 @@ __device__ __forceinline__ void icgn_solve(const IcgnParams& P, int64_t i, int l
     ++it;
     float A0 = 0.f, A1 = 0.f, A2 = 0.f, B[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     bool bad = false;
-    const bool lat = kSrc != kSrcCoefTile && (kSrc == kSrcPixels || P.lattice) && on_lattice(W, px, py);   // warp-uniform
+    const bool lat = kSrc != kSrcCoefTile && P.lattice && on_lattice(W, px, py);   // warp-uniform
     if constexpr (column_walk)
     {
-      bool fast = false;
-      if constexpr (kSrc == kSrcPixels)
-        fast = !lat && window_covers(W, px, py, rx, ry, xmax, ymax, T, lane);
-      if (fast)
-      {
-        if constexpr (kSrc == kSrcPixels)
-          if (col_active)
-          {
-            // every sample in range and in the window: no per-sample tests
-            const float ax = fmaf(W[0], flx_col, W[2]), ay = fmaf(W[3], flx_col, W[5]);
-            const int row = T.bx;
-            // (Loading the reference texel a row ahead of its use shortens the L2 waits but
-            // costs the registers that keep 32 warps resident: 3.27 against 2.94 ms.)
-            const float4* rp = ref_col;
-#pragma unroll kRowUnroll
-            for (int r = 0; r < 2 * ry + 1; ++r)
-            {
-              const float4 cur = __ldg(rp);
-              rp += w;
-              const float fly = (float)(r - ry);
-              const float gxp = px + fmaf(W[1], fly, ax);
-              const float gyp = py + fmaf(W[4], fly, ay);
-              const float t = sample_window(T, row, gxp, gyp);
-              const float tau = t - t0;
-              const float rc = cur.x - t0;
-              A0 += tau;
-              A1 = fmaf(tau, tau, A1);
-              A2 = fmaf(tau, rc, A2);
-              const float gt = __fmul_rn(cur.y, tau), ht = __fmul_rn(cur.z, tau);
-              B[0] = __fadd_rn(B[0], gt);
-              B[2] = fmaf(gt, fly, B[2]);
-              B[3] = __fadd_rn(B[3], ht);
-              B[5] = fmaf(ht, fly, B[5]);
-            }
-          }
-      }
-      else if (kSrc == kSrcPixels && col_active)
-      {
-        if constexpr (kSrc == kSrcPixels)
-        {
-          const ColumnSums c = px_column_checked(P.tar, w, h, T, ref_col, px, py, W[0], W[1], W[2], W[3], W[4], W[5],
-                                                 flx_col, t0, ry, lat ? 1 : 0);
-          A0 = c.A0;
-          A1 = c.A1;
-          A2 = c.A2;
-          B[0] = c.B0;
-          B[2] = c.B2;
-          B[3] = c.B3;
-          B[5] = c.B5;
-          bad = c.bad != 0;
-        }
-      }
-      else if (col_active)
+      if (col_active)
       {
         const float ax = fmaf(W[0], flx_col, W[2]), ay = fmaf(W[3], flx_col, W[5]);
 #pragma unroll kRowUnroll
@@ -1331,11 +1458,7 @@ __device__ __forceinline__ void icgn_solve(const IcgnParams& P, int64_t i, int l
           bad = true;
         else
         {
-          float t;
-          if constexpr (kSrc == kSrcPixels)
-            t = lat ? pixel_at(T, P.tar, px_pitch(w), gxp, gyp) : sample_pixels(T, P.tar, px_pitch(w), gxp, gyp);
-          else
-            t = lat ? __ldg(P.lattice + ((size_t)(int)gyp * w + (int)gxp)) : sample_bspline(coef, plane, w, gxp, gyp);
+          const float t = lat ? __ldg(P.lattice + ((size_t)(int)gyp * w + (int)gxp)) : sample_bspline(coef, plane, w, gxp, gyp);
           const float4 rv = __ldg(ref_pack + (size_t)(cy + ly) * w + (cx + lx));
           const float tau = t - t0;
           const float rc = rv.x - t0;
@@ -1451,6 +1574,10 @@ constexpr int icgn_min_blocks(int warps) { return DIC_ICGN_RESIDENT_WARPS / warp
 #define DIC_ICGN_PERSISTENT_RESIDENT_WARPS 32
 #endif
 constexpr int icgn_persistent_min_blocks(int warps) { return DIC_ICGN_PERSISTENT_RESIDENT_WARPS / warps; }
+// The pixel-window kernels: 20 resident warps (96 registers) for the column walk, 28 (72) for
+// the pair walk, whose windows leave room for no more above r 20.
+constexpr int px_min_blocks(int warps) { return 20 / warps; }
+constexpr int pair_px_min_blocks(int warps) { return 28 / warps; }
 
 template <bool kColumn, int kWarps = 4>
 __global__ void __launch_bounds__(kWarps * 32, icgn_min_blocks(kWarps)) k_icgn(IcgnParams P)
@@ -1558,68 +1685,26 @@ __device__ __forceinline__ bool pair_class_sums(const IcgnParams& P, int k, int 
   return any_bad;
 }
 
-// The same nine sums under pixel sampling (T: the POI's staged window).  `fast`: every sample of
-// the subset lies in the interpolation range and has its support in the window (window_covers,
-// once per iteration), so the rows run without tests; otherwise the checked loop of the column
-// walk (px_column_checked: range tests, window or global plane; `lat` on the pixel lattice).
-// Same sums in the same order as pair_class_sums, same bits in either loop.
+// The same nine sums under pixel sampling (T: the POI's staged window), by px_column.  `covered`:
+// every sample of the subset lies in the interpolation range and has its support in the window
+// (window_covers, once per iteration); `lat`: on the pixel lattice.
 __device__ __forceinline__ bool pair_class_sums_px(const IcgnParams& P, const PixelTile& T, int k, int lane, float px,
-                                                   float py, int cx, int cy, float t0, const float (&W)[6], bool fast,
+                                                   float py, int cx, int cy, float t0, const float (&W)[6], bool covered,
                                                    bool lat, float (&s)[9])
 {
   const int rx = P.rx, ry = P.ry, w = P.w;
   const int c = pair_column(lane, k);
   const float flx = (float)(c - rx);
-  float A0 = 0.f, A1 = 0.f, A2 = 0.f, B[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  bool bad = false;
+  const unsigned mask = __ballot_sync(kFull, c < 2 * rx + 1);
+  ColumnSums cs{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
   if (c < 2 * rx + 1)
-  {
-    const float4* __restrict__ ref_col = P.ref_pack + (size_t)(cy - ry) * w + cx + (c - rx);
-    if (fast)
-    {
-      const float ax = fmaf(W[0], flx, W[2]), ay = fmaf(W[3], flx, W[5]);
-      const int row = T.bx;
-      const float4* rp = ref_col;
-      const auto accumulate = [&](float t, const float4& cur, float fly) {
-        const float tau = t - t0;
-        const float rc = cur.x - t0;
-        A0 += tau;
-        A1 = fmaf(tau, tau, A1);
-        A2 = fmaf(tau, rc, A2);
-        const float gt = __fmul_rn(cur.y, tau), ht = __fmul_rn(cur.z, tau);
-        B[0] = __fadd_rn(B[0], gt);
-        B[2] = fmaf(gt, fly, B[2]);
-        B[3] = __fadd_rn(B[3], ht);
-        B[5] = fmaf(ht, fly, B[5]);
-      };
-      for (int r = 0; r < 2 * ry + 1; ++r)
-      {
-        const float4 cur = __ldg(rp);
-        rp += w;
-        const float fly = (float)(r - ry);
-        accumulate(sample_window(T, row, px + fmaf(W[1], fly, ax), py + fmaf(W[4], fly, ay)), cur, fly);
-      }
-    }
-    else
-    {
-      const ColumnSums cs = px_column_checked(P.tar, w, P.h, T, ref_col, px, py, W[0], W[1], W[2], W[3], W[4], W[5],
-                                              flx, t0, ry, lat ? 1 : 0);
-      A0 = cs.A0;
-      A1 = cs.A1;
-      A2 = cs.A2;
-      B[0] = cs.B0;
-      B[2] = cs.B2;
-      B[3] = cs.B3;
-      B[5] = cs.B5;
-      bad = cs.bad != 0;
-    }
-  }
-  B[1] = flx * B[0];
-  B[4] = flx * B[3];
-  const bool any_bad = __any_sync(kFull, bad);
-  s[0] = warp_sum(A0);
-  s[1] = warp_sum(A1);
-  s[2] = warp_sum(A2);
+    cs = px_column(T, P.tar, P.ref_pack + (size_t)(cy - ry) * w + cx + (c - rx), w, P.h, px, py, W, flx, t0, ry, covered,
+                   lat, mask);
+  const bool any_bad = __any_sync(kFull, cs.bad != 0);
+  s[0] = warp_sum(cs.A0);
+  s[1] = warp_sum(cs.A1);
+  s[2] = warp_sum(cs.A2);
+  const float B[6] = {cs.B0, flx * cs.B0, cs.B2, cs.B3, flx * cs.B3, cs.B5};
 #pragma unroll
   for (int a = 0; a < 6; ++a) s[3 + a] = warp_sum(B[a]);
   return any_bad;
@@ -1689,16 +1774,16 @@ __device__ __forceinline__ void icgn_solve_pair(const IcgnParams& P, int64_t i, 
     ++it;
     float s[9];
     bool bad;
-    // pixel sampling: on the lattice, or every sample inside the window (warp-uniform)
-    bool fast = false, lat = false;
+    // pixel sampling: on the lattice, every sample inside the window (warp-uniform)
+    bool covered = false, lat = false;
     if constexpr (kSrc == kSrcPixels)
     {
       lat = on_lattice(W, px, py);
-      fast = !lat && window_covers(W, px, py, rx, ry, (float)(w - 2), (float)(h - 2), T, lane);
+      covered = window_covers(W, px, py, rx, ry, (float)(w - 2), (float)(h - 2), T, lane);
     }
     const auto class_sums = [&](int k, float(&out)[9]) {
       if constexpr (kSrc == kSrcPixels)
-        return pair_class_sums_px(P, T, k, lane, px, py, cx, cy, t0, W, fast, lat, out);
+        return pair_class_sums_px(P, T, k, lane, px, py, cx, cy, t0, W, covered, lat, out);
       else
         return pair_class_sums(P, k, lane, px, py, cx, cy, t0, W, out);
     };
@@ -2033,10 +2118,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
 // (bounded) for the copy still in flight, and leaves.
 // --------------------------------------------------------------------------------------
 constexpr int kPxMargin = 1;
-#ifndef DIC_PX_ROW_UNROLL
-#define DIC_PX_ROW_UNROLL 1
-#endif
-constexpr int kPxRowUnroll = DIC_PX_ROW_UNROLL;   // rows of the pixel walk unrolled together
 
 // window of one warp for a subset radius: the support of the subset with the margin and
 // the x alignment slack, x rounded up to a multiple of 4 pixels
@@ -2176,12 +2257,162 @@ __device__ __forceinline__ int px_window(int warp, size_t win_bytes, uint32_t& a
   return (int)(off / sizeof(float));
 }
 
+// The nine sums of the lanes in an xor butterfly's order (the same pairings as warp_sum, so the
+// same bits) with a third of its shuffles: eight values are halved across the lanes on the way
+// (each lane keeps the half its bit 4, 3, 2 selects), which leaves value v of {B0..B5, A1, A2} on
+// lanes 4 v .. 4 v + 3; A0 is summed on every lane.
+__device__ __forceinline__ float reduce_sums(const ColumnSums& c, float flx, int lane, float& A0, float& A1, float& A2)
+{
+  const float v[8] = {c.B0, flx * c.B0, c.B2, c.B3, flx * c.B3, c.B5, c.A1, c.A2};
+  const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+  float x[4], y[2];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) x[j] = (b4 ? v[j + 4] : v[j]) + __shfl_xor_sync(kFull, b4 ? v[j] : v[j + 4], 16);
+#pragma unroll
+  for (int j = 0; j < 2; ++j) y[j] = (b3 ? x[j + 2] : x[j]) + __shfl_xor_sync(kFull, b3 ? x[j] : x[j + 2], 8);
+  float z = (b2 ? y[1] : y[0]) + __shfl_xor_sync(kFull, b2 ? y[0] : y[1], 4);
+  z += __shfl_xor_sync(kFull, z, 2);
+  z += __shfl_xor_sync(kFull, z, 1);
+  A0 = warp_sum(c.A0);
+  A1 = __shfl_sync(kFull, z, 24);
+  A2 = __shfl_sync(kFull, z, 28);
+  return z;
+}
+
+// PoiRef as floats in shared memory, one copy per POI in flight: every iteration reads it, and
+// from global memory those reads missed L1 (9 % hit rate: the reference rows of 32 POIs pass
+// through it), an L2 round trip per iteration and warp.
+constexpr int kRefFloats = sizeof(PoiRef) / sizeof(float);
+constexpr int kRefNorm = offsetof(PoiRef, ref_norm) / 4, kRefNormSq = offsetof(PoiRef, ref_norm_sq) / 4,
+              kRefSumRc = offsetof(PoiRef, sum_rc) / 4, kRefS = offsetof(PoiRef, S) / 4, kRefG = offsetof(PoiRef, G) / 4,
+              kRefInvH = offsetof(PoiRef, inv_h) / 4;
+
+// One POI (queue index i) on the calling warp under pixel sampling, column walk: icgn_solve's
+// rules, codes and outputs from the staged window T.  ref: the warp's copy of the POI's record.
+__device__ __forceinline__ void icgn_solve_px(const IcgnParams& P, int64_t i, int lane, const PixelTile& T,
+                                              const float* ref)
+{
+  dic_poi* poi = P.pois + i;
+  const float px = poi->x, py = poi->y;
+  const float u_in = poi->u, ux_in = poi->ux, uy_in = poi->uy;
+  const float v_in = poi->v, vx_in = poi->vx, vy_in = poi->vy;
+  const float zncc_in = poi->zncc;
+  const int w = P.w, h = P.h, rx = P.rx, ry = P.ry;
+  // Entry test (src/oc_icgn.cpp:184-191).
+  if (py - ry < 0 || px - rx < 0 || py + ry > h - 1 || px + rx > w - 1 || fabsf(u_in) >= w ||
+      fabsf(v_in) >= h || zncc_in < 0 || isnan(u_in) || isnan(v_in))
+  {
+    if (lane == 0) poi->zncc = zncc_in >= 0 ? -3.f : zncc_in;
+    return;
+  }
+  const float t0 = ref[0];
+  const int sw = 2 * rx + 1;
+  const float inv_size = 1.f / (float)(sw * (2 * ry + 1));
+  float W[6] = {1.f + ux_in, uy_in, u_in, vx_in, 1.f + vy_in, v_in};
+  const float rx2 = (float)(rx * rx), ry2 = (float)(ry * ry);
+  const float xmax = (float)(w - 2), ymax = (float)(h - 2);
+  const bool col_active = lane < sw;
+  const float flx = (float)(lane - rx);
+  const unsigned mask = sw >= 32 ? kFull : (1u << sw) - 1u;
+  const float4* ref_col = P.ref_pack + (size_t)((int)py - ry) * w + (int)px + (lane - rx);
+  int it = 0;
+  float conv = 0.f, s = 0.f, tnorm_sq = 0.f, tc_rc = 0.f;
+  int status = 0;  // 0 ok, -3 out of range, -5 NaN coordinate
+  do
+  {
+    ++it;
+    ColumnSums c{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
+    const bool covered = window_covers(W, px, py, rx, ry, xmax, ymax, T, lane);
+    if (col_active) c = px_column(T, P.tar, ref_col, w, h, px, py, W, flx, t0, ry, covered, on_lattice(W, px, py), mask);
+    if (__any_sync(kFull, c.bad))
+    {
+      // Rare path: classify with the CPU's order (src/oc_icgn.cpp:266-301).
+      bool oob = false;
+      if (col_active)
+      {
+        const float ax = fmaf(W[0], flx, W[2]), ay = fmaf(W[3], flx, W[5]);
+        for (int r = 0; r < 2 * ry + 1; ++r)
+        {
+          const float fly = (float)(r - ry);
+          const float gxp = px + fmaf(W[1], fly, ax), gyp = py + fmaf(W[4], fly, ay);
+          if (gxp < 1.f || gyp < 1.f || gxp >= xmax || gyp >= ymax) oob = true;
+        }
+      }
+      status = __any_sync(kFull, oob) ? -3 : -5;
+      break;
+    }
+    float A0, A1, A2;
+    const float b = reduce_sums(c, flx, lane, A0, A1, A2);   // B of row lane / 4
+    const float ref_norm = ref[kRefNorm];
+    const float mean_tau = A0 * inv_size;
+    tnorm_sq = fmaf(-A0, mean_tau, A1);
+    // A flat target subset has zero norm; the CPU then divides by zero and the POI ends
+    // as NaN (-5).  Rounding can leave a tiny residue here, so force the same outcome.
+    const float tar_norm = tnorm_sq > 0.f ? sqrtf(tnorm_sq) : __int_as_float(0x7fc00000);
+    s = ref_norm / tar_norm;
+    tc_rc = fmaf(-mean_tau, ref[kRefSumRc], A2);
+    // rows a = lane / 4 < 6: num_a, then dp_a = invH row a . num
+    const int row = lane < 24 ? lane >> 2 : 0;
+    const float num = s * fmaf(-mean_tau, ref[kRefS + row], b) - ref[kRefG + row];
+    float dp_l = 0.f;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) dp_l += ref[kRefInvH + row * 6 + k] * __shfl_sync(kFull, num, 4 * k);
+    float dp[6];
+#pragma unroll
+    for (int a = 0; a < 6; ++a) dp[a] = __shfl_sync(kFull, dp_l, 4 * a);
+    compose_update(W, dp);
+    conv = sqrtf(dp[0] * dp[0] + dp[1] * dp[1] * rx2 + dp[2] * dp[2] * ry2 + dp[3] * dp[3] +
+                 dp[4] * dp[4] * rx2 + dp[5] * dp[5] * ry2);
+  } while ((float)it < P.max_iter && conv >= P.conv);
+
+  if (lane != 0) return;
+  if (P.iter_sum) atomicAdd(P.iter_sum, (unsigned long long)it);
+  if (status == -3) { poi->zncc = -3.f; return; }   // src/oc_icgn.cpp:285-289
+  if (status == -5) { poi->zncc = -5.f; return; }   // :297-301
+  const float ref_norm = ref[kRefNorm];
+  const float esq = s * s * tnorm_sq - 2.f * s * tc_rc + ref[kRefNormSq];
+  const float znssd = esq / (ref_norm * ref_norm);
+  float u = W[2], v = W[5];
+  float zncc = 0.5f * (2.f - znssd);
+  if (conv >= P.conv && (float)it >= P.max_iter) zncc = -4.f;
+  // The incoming guess is re-read here (the record is still unmodified) rather than kept
+  // live across the iteration loop.
+  const float u_init = poi->u, v_init = poi->v;
+  if (isnan(zncc) || isnan(u) || isnan(v))
+  {
+    u = u_init;
+    v = v_init;
+    zncc = -5.f;
+  }
+  poi->u = u; poi->ux = W[0] - 1.f; poi->uy = W[1];
+  poi->v = v; poi->vx = W[3]; poi->vy = W[4] - 1.f;
+  poi->u0 = u_init;
+  poi->v0 = v_init;
+  poi->zncc = zncc;
+  poi->iteration = (float)it;
+  poi->convergence = conv;
+}
+
+// The POI's reference record on its way to the warp's copy: two floats on lanes 0-27, loaded
+// before the window's copy is waited for and stored after it.
+__device__ __forceinline__ float2 ref_fetch(const IcgnParams& P, int64_t i, int lane)
+{
+  const float2* r = reinterpret_cast<const float2*>(P.poi_ref + (P.slot ? P.slot[i] : i));
+  return lane < kRefFloats / 2 ? __ldg(r + lane) : make_float2(0.f, 0.f);
+}
+__device__ __forceinline__ void ref_store(float* ref, float2 v, int lane)
+{
+  if (lane < kRefFloats / 2) reinterpret_cast<float2*>(ref)[lane] = v;
+  __syncwarp();
+}
+
 // kMode: 2 windows staged by TMA, 1 staged by warp copies, 0 no windows (every sample from
 // the global plane)
 template <int kWarps, int kMode>
-__global__ void __launch_bounds__(kWarps * 32, icgn_persistent_min_blocks(kWarps))
+__global__ void __launch_bounds__(kWarps * 32, px_min_blocks(kWarps))
     k_icgn_px(IcgnParams P, const __grid_constant__ CUtensorMap map, unsigned long long* next, int* err)
 {
+  __shared__ __align__(16) float refs[kWarps][kRefFloats];
   __shared__ __align__(8) unsigned long long bars[kWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (P.enable && *P.enable == 0) return;
@@ -2198,8 +2429,10 @@ __global__ void __launch_bounds__(kWarps * 32, icgn_persistent_min_blocks(kWarps
     const int64_t i = (int64_t)__shfl_sync(kFull, t, 0);
     if (!queue_slot_active(P, i)) return;
     PixelTile T;
+    const float2 rv = ref_fetch(P, i, lane);
     if (!px_stage<kMode>(P, i, lane, win_f, win, &map, bar, parity, err, T)) return;
-    icgn_solve<true, kSrcPixels, kPxRowUnroll, PixelTile>(P, i, lane, T);
+    ref_store(refs[warp], rv, lane);
+    icgn_solve_px(P, i, lane, T, refs[warp]);
     __syncwarp();   // every lane's reads of this window before the next copy overwrites it
   }
 }
@@ -2231,7 +2464,7 @@ __device__ __forceinline__ int64_t pair_fetch(unsigned long long* next, long lon
 // kMode as in k_icgn_px (2 TMA, 1 warp copies, 0 no windows).  Same bits for every kPoiWarps,
 // kWarps and kMode.
 template <int kPoiWarps, int kWarps, int kMode>
-__global__ void __launch_bounds__(kWarps * 32, icgn_min_blocks(kWarps))
+__global__ void __launch_bounds__(kWarps * 32, pair_px_min_blocks(kWarps))
     k_icgn_pair_px(IcgnParams P, const __grid_constant__ CUtensorMap map, unsigned long long* next, int* err)
 {
   constexpr int kSlots = kWarps / kPoiWarps;
@@ -2339,11 +2572,12 @@ __device__ __forceinline__ int batch_job_of(const BatchJob* __restrict__ jobs, i
 // kMode 2: every job has a map (TMA windows); 1: warp copies for all.  32 resident warps per
 // SM (64 registers, no spills), as k_icgn_px.
 template <int kWarps, int kMode>
-__global__ void __launch_bounds__(kWarps * 32, icgn_persistent_min_blocks(kWarps))
+__global__ void __launch_bounds__(kWarps * 32, px_min_blocks(kWarps))
     k_icgn_batch_px(const BatchJob* __restrict__ jobs, int njobs, dic_poi* pois, const PoiRef* poi_ref, int64_t begin,
                     int64_t end, unsigned long long* next, float conv, float max_iter, unsigned long long* iter_sum,
                     uint32_t win_bytes, uint32_t wait_polls, int* err)
 {
+  __shared__ __align__(16) float refs[kWarps][kRefFloats];
   __shared__ __align__(8) unsigned long long bars[kWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t win = 0, parity = 0;
@@ -2375,8 +2609,10 @@ __global__ void __launch_bounds__(kWarps * 32, icgn_persistent_min_blocks(kWarps
     P.iter_sum = iter_sum;
     P.wait_polls = wait_polls;
     PixelTile T;
+    const float2 rv = ref_fetch(P, k, lane);
     if (!px_stage<kMode>(P, k, lane, win_f, win, J.map, bar, parity, err, T)) return;
-    icgn_solve<true, kSrcPixels, 1, PixelTile>(P, k, lane, T);
+    ref_store(refs[warp], rv, lane);
+    icgn_solve_px(P, k, lane, T, refs[warp]);
     __syncwarp();
   }
 }
@@ -2434,7 +2670,7 @@ __global__ void __launch_bounds__(kWarps * 32, icgn_min_blocks(kWarps))
 // k_icgn_pair_px's windows (each job's map in device memory, win_bytes the window of the
 // launch's largest radius).  kMode 2: TMA windows (every job has a map), 0: no windows.
 template <int kPoiWarps, int kWarps, int kMode>
-__global__ void __launch_bounds__(kWarps * 32, icgn_min_blocks(kWarps))
+__global__ void __launch_bounds__(kWarps * 32, pair_px_min_blocks(kWarps))
     k_icgn_batch_pair_px(const BatchJob* __restrict__ jobs, int njobs, dic_poi* pois, const PoiRef* poi_ref,
                          int64_t begin, int64_t end, unsigned long long* next, float conv, float max_iter,
                          unsigned long long* iter_sum, uint32_t win_bytes, uint32_t wait_polls, int* err)
@@ -2490,16 +2726,6 @@ __global__ void __launch_bounds__(kWarps * 32, icgn_min_blocks(kWarps))
 // later; each half rounded as the scalar operation): the FFTCC line transforms issue half the
 // instructions for their butterflies (k_fftcc2<30> 0.756 -> 0.674 ms on the 2048x2048 pair).
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b)
-{
-  unsigned long long ra, rb, rd;
-  memcpy(&ra, &a, 8);
-  memcpy(&rb, &b, 8);
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(rd) : "l"(ra), "l"(rb));
-  float2 d;
-  memcpy(&d, &rd, 8);
-  return d;
-}
 __device__ __forceinline__ float2 cscale(float2 a, float s) { return __fmul2_rn(a, make_float2(s, s)); }
 __device__ __forceinline__ float2 cmul(float2 a, float2 b)
 { return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
