@@ -12,10 +12,9 @@
 //
 // Activations are BF16 in NHWC order (channels fastest), weights are kept in FP32 (master)
 // with BF16 working copies, and every product runs on the tensor cores with FP32
-// accumulation.  Training: one GEMM kernel (mma.sync.m16n8k16 bf16) serves all layers and
-// passes; an operand functor gathers its A and B tiles (implicit im2col for the
-// convolutions) and an epilogue functor stores the result.  Inference (k_proposal_fused)
-// runs conv2, its largest layer, as tcgen05.mma from shared-memory descriptors into TMEM.
+// accumulation.  Training runs layer by layer (dic_cnn_train.cuh).  Inference
+// (k_proposal_fused) runs conv2, its largest layer, as tcgen05.mma from shared-memory
+// descriptors into TMEM.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -74,253 +73,7 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], const uint32_t (&a
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// --------------------------------------------------------------------------------------
-// Generic GEMM: C[M x N] = A[M x K] * B[K x N] over k in [k_lo, k_hi) of this split.
-// CTA tile 64 x 32 x 32, 4 warps, each warp 16 rows x 32 columns (four m16n8k16 per
-// k16 step).  Op supplies M, N, K, splits, a(m, k), b(k, n) (BF16, 0 outside), and
-// store(split, m, n, value) for the FP32 accumulator.
-// --------------------------------------------------------------------------------------
-constexpr int BM = 64, BN = 32, BK = 32;
-
-template <class Op>
-__global__ void __launch_bounds__(128) k_gemm(Op op)
-{
-  __shared__ __nv_bfloat16 As[BM][BK + 8];
-  __shared__ __nv_bfloat16 Bs[BN][BK + 8];
-  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-  const int split = blockIdx.z;
-  const int64_t kper = ((op.K + BK - 1) / BK + op.splits - 1) / op.splits * BK;
-  const int64_t k_lo = (int64_t)split * kper;
-  const int64_t k_hi = k_lo + kper < op.K ? k_lo + kper : op.K;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
-  float acc[4][4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) acc[j][q] = 0.f;
-  for (int64_t k0 = k_lo; k0 < k_hi; k0 += BK)
-  {
-    for (int e = threadIdx.x; e < BM * BK; e += blockDim.x)
-    {
-      const int r = e / BK, c = e % BK;
-      const int64_t k = k0 + c;
-      As[r][c] = (k < k_hi) ? op.a(m0 + r, k) : __float2bfloat16(0.f);
-    }
-    for (int e = threadIdx.x; e < BN * BK; e += blockDim.x)
-    {
-      const int r = e / BK, c = e % BK;
-      const int64_t k = k0 + c;
-      Bs[r][c] = (k < k_hi) ? op.b(k, n0 + r) : __float2bfloat16(0.f);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < BK; kk += 16)
-    {
-      const int r = warp * 16 + g, c = kk + t4 * 2;
-      uint32_t a[4];
-      a[0] = pack_bf16(As[r][c], As[r][c + 1]);
-      a[1] = pack_bf16(As[r + 8][c], As[r + 8][c + 1]);
-      a[2] = pack_bf16(As[r][c + 8], As[r][c + 9]);
-      a[3] = pack_bf16(As[r + 8][c + 8], As[r + 8][c + 9]);
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-      {
-        const int nn = j * 8 + g;
-        uint32_t b[2];
-        b[0] = pack_bf16(Bs[nn][c], Bs[nn][c + 1]);
-        b[1] = pack_bf16(Bs[nn][c + 8], Bs[nn][c + 9]);
-        mma_bf16_16816(acc[j], a, b);
-      }
-    }
-    __syncthreads();
-  }
-  const int r0 = m0 + warp * 16 + g;
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-  {
-    const int c = n0 + j * 8 + t4 * 2;
-    op.store(split, r0, c, acc[j][0]);
-    op.store(split, r0, c + 1, acc[j][1]);
-    op.store(split, r0 + 8, c, acc[j][2]);
-    op.store(split, r0 + 8, c + 1, acc[j][3]);
-  }
-}
-
 __device__ __forceinline__ __nv_bfloat16 bz() { return __float2bfloat16(0.f); }
-
-// Convolution geometry: input side si, channels ci; output side so = si / 2 rounded up
-// (3x3, stride 2, pad 1).  Activations NHWC: act[((n * s + y) * s + x) * c + ch].
-struct ConvGeom
-{
-  int si, so, ci, co;
-  int kdim() const { return 9 * ci; }
-};
-
-// Forward: A[m = (n, oy, ox)][k = (ky, kx, ci)] = in[n, 2oy+ky-1, 2ox+kx-1, ci],
-// B[k][n = co] = W[co][k]; store z + bias, ReLU, BF16.
-struct ConvFwdOp
-{
-  const __nv_bfloat16* in;
-  const __nv_bfloat16* w;   // [co][kpad]
-  const float* bias;
-  __nv_bfloat16* out;
-  int64_t M;
-  int N, splits;
-  int64_t K;                // padded K
-  int si, so, ci, kreal, kpad;
-  __device__ __nv_bfloat16 a(int64_t m, int64_t k) const
-  {
-    if (m >= M || k >= kreal) return bz();
-    const int64_t n = m / (so * so);
-    const int p = (int)(m % (so * so)), oy = p / so, ox = p % so;
-    const int c = (int)(k % ci), kk = (int)(k / ci), ky = kk / 3, kx = kk % 3;
-    const int iy = 2 * oy + ky - 1, ix = 2 * ox + kx - 1;
-    if (iy < 0 || ix < 0 || iy >= si || ix >= si) return bz();
-    return in[((n * si + iy) * si + ix) * ci + c];
-  }
-  __device__ __nv_bfloat16 b(int64_t k, int n) const { return n < N ? w[(int64_t)n * kpad + k] : bz(); }
-  __device__ void store(int, int64_t m, int n, float v) const
-  {
-    if (m >= M || n >= N) return;
-    out[m * N + n] = __float2bfloat16(fmaxf(v + bias[n], 0.f));
-  }
-};
-
-// Backward data: dIn[m = (n, iy, ix)][c] = sum over (ky, kx, co) of
-// dZ[n, oy, ox, co] W[co][ky][kx][c] with iy = 2oy+ky-1; then the ReLU mask of the input
-// activation (act > 0), stored BF16 as the previous layer's dZ.
-struct ConvBwdDataOp
-{
-  const __nv_bfloat16* dz;    // [N][so][so][co]
-  const __nv_bfloat16* w;     // [co][kpad], k = (ky, kx, ci)
-  const __nv_bfloat16* act;   // input activation [N][si][si][ci] (ReLU output)
-  __nv_bfloat16* dzin;        // [N][si][si][ci]
-  int64_t M;
-  int N, splits;
-  int64_t K;                  // 9 * co
-  int si, so, ci, co, kpad;
-  __device__ __nv_bfloat16 a(int64_t m, int64_t k) const
-  {
-    if (m >= M || k >= K) return bz();
-    const int64_t n = m / (si * si);
-    const int p = (int)(m % (si * si)), iy = p / si, ix = p % si;
-    const int o = (int)(k % co), kk = (int)(k / co), ky = kk / 3, kx = kk % 3;
-    const int ty = iy + 1 - ky, tx = ix + 1 - kx;
-    if (ty < 0 || tx < 0 || (ty & 1) || (tx & 1)) return bz();
-    const int oy = ty >> 1, ox = tx >> 1;
-    if (oy >= so || ox >= so) return bz();
-    return dz[((n * so + oy) * so + ox) * co + o];
-  }
-  __device__ __nv_bfloat16 b(int64_t k, int c) const
-  {
-    if (c >= N || k >= K) return bz();
-    const int o = (int)(k % co), kk = (int)(k / co);
-    return w[(int64_t)o * kpad + kk * ci + c];
-  }
-  __device__ void store(int, int64_t m, int c, float v) const
-  {
-    if (m >= M || c >= N) return;
-    const int64_t i = m * N + c;
-    dzin[i] = __float2bfloat16(__bfloat162float(act[i]) > 0.f ? v : 0.f);
-  }
-};
-
-// Backward weights: dW[co][k = (ky, kx, ci)] = sum over (n, oy, ox) of dZ[n, oy, ox, co] *
-// in[n, 2oy+ky-1, 2ox+kx-1, ci]; split-K partials go to part[split][co][kpad] (FP32) and
-// k_reduce_splits sums them in a fixed order.
-struct ConvBwdWeightOp
-{
-  const __nv_bfloat16* dz;    // [Nb][so][so][co]
-  const __nv_bfloat16* in;    // [Nb][si][si][ci]
-  float* part;
-  int64_t M;                  // co
-  int N, splits;              // N = kpad columns
-  int64_t K;                  // Nb * so * so
-  int si, so, ci, co, kreal, kpad;
-  __device__ __nv_bfloat16 a(int64_t m, int64_t k) const
-  {
-    if (m >= M || k >= K) return bz();
-    return dz[k * co + m];
-  }
-  __device__ __nv_bfloat16 b(int64_t k, int col) const
-  {
-    if (col >= kreal || k >= K) return bz();
-    const int64_t n = k / (so * so);
-    const int p = (int)(k % (so * so)), oy = p / so, ox = p % so;
-    const int c = col % ci, kk = col / ci, ky = kk / 3, kx = kk % 3;
-    const int iy = 2 * oy + ky - 1, ix = 2 * ox + kx - 1;
-    if (iy < 0 || ix < 0 || iy >= si || ix >= si) return bz();
-    return in[((n * si + iy) * si + ix) * ci + c];
-  }
-  __device__ void store(int split, int64_t m, int col, float v) const
-  {
-    if (m >= M || col >= N) return;
-    part[((int64_t)split * M + m) * N + col] = v;
-  }
-};
-
-// Dense forward: out[m][n] = act(sum_k in[m][k] W[n][k] + bias[n]).
-struct LinearFwdOp
-{
-  const __nv_bfloat16* in;    // [M][K]
-  const __nv_bfloat16* w;     // [Npad][K]
-  const float* bias;
-  __nv_bfloat16* out_bf;      // ReLU layer output (nullable)
-  float* out_f;               // linear output (nullable), [M][ld]
-  int64_t M;
-  int N, splits;
-  int64_t K;
-  int ld;
-  __device__ __nv_bfloat16 a(int64_t m, int64_t k) const { return m < M ? in[m * K + k] : bz(); }
-  __device__ __nv_bfloat16 b(int64_t k, int n) const { return n < N ? w[(int64_t)n * K + k] : bz(); }
-  __device__ void store(int, int64_t m, int n, float v) const
-  {
-    if (m >= M || n >= N) return;
-    const float z = v + bias[n];
-    if (out_bf) out_bf[m * N + n] = __float2bfloat16(fmaxf(z, 0.f));
-    if (out_f) out_f[m * ld + n] = z;
-  }
-};
-
-// Dense backward data: dIn[m][k] = sum_n dZ[m][n] W[n][k], masked by act[m][k] > 0.
-struct LinearBwdDataOp
-{
-  const __nv_bfloat16* dz;    // [M][Nout]
-  const __nv_bfloat16* w;     // [Npad][Kin]
-  const __nv_bfloat16* act;   // [M][Kin]
-  __nv_bfloat16* dzin;        // [M][Kin]
-  int64_t M;
-  int N, splits;              // N = Kin
-  int64_t K;                  // Nout
-  int nout_pad;
-  __device__ __nv_bfloat16 a(int64_t m, int64_t k) const { return (m < M && k < K) ? dz[m * nout_pad + k] : bz(); }
-  __device__ __nv_bfloat16 b(int64_t k, int c) const { return (c < N && k < K) ? w[k * N + c] : bz(); }
-  __device__ void store(int, int64_t m, int c, float v) const
-  {
-    if (m >= M || c >= N) return;
-    const int64_t i = m * N + c;
-    dzin[i] = __float2bfloat16(__bfloat162float(act[i]) > 0.f ? v : 0.f);
-  }
-};
-
-// Dense backward weights: dW[n][k] = sum_m dZ[m][n] in[m][k]; split-K partials.
-struct LinearBwdWeightOp
-{
-  const __nv_bfloat16* dz;    // [Mb][ldz]
-  const __nv_bfloat16* in;    // [Mb][Kin]
-  float* part;                // [split][Nout][Kin]
-  int64_t M;                  // Nout
-  int N, splits;              // Kin
-  int64_t K;                  // batch
-  int ldz;
-  __device__ __nv_bfloat16 a(int64_t m, int64_t k) const { return (m < M && k < K) ? dz[k * ldz + m] : bz(); }
-  __device__ __nv_bfloat16 b(int64_t k, int c) const { return (c < N && k < K) ? in[k * N + c] : bz(); }
-  __device__ void store(int split, int64_t m, int c, float v) const
-  {
-    if (m >= M || c >= N) return;
-    part[((int64_t)split * M + m) * N + c] = v;
-  }
-};
 
 // --------------------------------------------------------------------------------------
 // Element kernels
@@ -402,61 +155,6 @@ __global__ void k_pack_weights(const float* __restrict__ p, __nv_bfloat16* __res
 // Output scaling: the network predicts (u, v, 100 ux, 100 uy, 100 vx, 100 vy).
 __host__ __device__ constexpr float out_scale(int j) { return j < 2 ? 1.f : 100.f; }
 
-// MSE over the six scaled outputs, mean over batch and outputs.  dout = dL/dout (BF16),
-// per-row loss partial into row_loss (summed on the host side in a fixed order).
-__global__ void k_loss_grad(const float* __restrict__ out, const float* __restrict__ target, int64_t n,
-                            __nv_bfloat16* __restrict__ dout, float* __restrict__ row_loss)
-{
-  const int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= n) return;
-  float l = 0.f;
-  const float scale = 2.f / (float)(n * kOut);
-#pragma unroll
-  for (int j = 0; j < kOutPad; ++j)
-  {
-    float g = 0.f;
-    if (j < kOut)
-    {
-      const float d = out[m * kOutPad + j] - target[m * kOut + j] * out_scale(j);
-      l += d * d;
-      g = d * scale;
-    }
-    dout[m * kOutPad + j] = __float2bfloat16(g);
-  }
-  row_loss[m] = l;
-}
-
-// Bias gradient: db[c] = sum over rows of dz[row][c] (BF16 rows of width ld), fixed order.
-__global__ void k_bias_grad(const __nv_bfloat16* __restrict__ dz, int64_t rows, int ld, int ncol, float* __restrict__ db)
-{
-  const int c = blockIdx.x;
-  if (c >= ncol) return;
-  float s = 0.f;
-  for (int64_t r = threadIdx.x; r < rows; r += blockDim.x) s += __bfloat162float(dz[r * ld + c]);
-  __shared__ float red[256];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1)
-  {
-    if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) db[c] = red[0];
-}
-
-// Sum split-K partials part[s][rows][cols] in split order into out[r * out_ld + c] for
-// c < keep (the unpadded columns).
-__global__ void k_reduce_splits(const float* __restrict__ part, int splits, int rows, int cols, int keep,
-                                float* __restrict__ out, int out_ld)
-{
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rows * keep) return;
-  const int r = i / keep, c = i % keep;
-  float s = 0.f;
-  for (int k = 0; k < splits; ++k) s += part[((int64_t)k * rows + r) * cols + c];
-  out[(int64_t)r * out_ld + c] = s;
-}
-
 // Adam (Kingma & Ba 2015) on the FP32 master parameters.
 __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
                        int n, float lr, float b1, float b2, float eps, float c1, float c2)
@@ -469,23 +167,6 @@ __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float
   m[i] = mi;
   v[i] = vi;
   p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-}
-
-// Network output -> queue seed (u, ux, uy, v, vx, vy); result fields cleared.
-__global__ void k_write_seeds(const float* __restrict__ out, dic_poi* __restrict__ pois, int64_t n)
-{
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float* o = out + i * kOutPad;
-  dic_poi q = pois[i];
-  q.u = o[0];
-  q.v = o[1];
-  q.ux = o[2] / out_scale(2);
-  q.uy = o[3] / out_scale(3);
-  q.vx = o[4] / out_scale(4);
-  q.vy = o[5] / out_scale(5);
-  q.u0 = 0.f; q.v0 = 0.f; q.zncc = 0.f; q.iteration = 0.f; q.convergence = 0.f; q.feature = 0.f;
-  pois[i] = q;
 }
 
 // --------------------------------------------------------------------------------------
@@ -1115,3 +796,5 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
 
 }  // namespace cnn
 }  // namespace dic
+
+#include "dic_cnn_train.cuh"

@@ -112,7 +112,7 @@ enum Phase { kPhRef = 0, kPhPoi, kPhTar, kPhFftcc, kPhIcgn, kPhFrame, kPhProposa
 // ======================================================================================
 struct dic_cnn
 {
-  int device = 0;
+  int device = 0, sms = 0;
   cudaStream_t stream = nullptr;   // own stream; an engine borrows the network on its stream
   std::string last_error;
   DevBuf<float> params, grads, adam_m, adam_v, out, part, row_loss;
@@ -152,115 +152,73 @@ struct dic_cnn
     check("k_pack_weights");
   }
 
-  template <class Op>
-  void gemm(const Op& op, int64_t m_rows, int n_cols)
+  // CTAs of 256 threads (eight 16-row tiles) for a layer's rows, at most `per_sm` per SM
+  unsigned tile_grid(int64_t rows, int per_sm) const
   {
-    dim3 grid((unsigned)((m_rows + cnn::BM - 1) / cnn::BM), (unsigned)((n_cols + cnn::BN - 1) / cnn::BN),
-              (unsigned)op.splits);
-    cnn::k_gemm<Op><<<grid, 128, 0, stream>>>(op);
-    check("k_gemm");
+    return (unsigned)std::min<int64_t>((rows + 127) / 128, (int64_t)sms * per_sm);
+  }
+  // The layers read x0 as 4-byte pixels; an input that starts between them is copied first.
+  const uint32_t* pixels(const void* in, int64_t n)
+  {
+    if ((reinterpret_cast<uintptr_t>(in) & 3) == 0) return static_cast<const uint32_t*>(in);
+    DIC_CUDA(cudaMemcpyAsync(x0.ptr, in, (size_t)n * cnn::kWin * cnn::kWin * 4, cudaMemcpyDeviceToDevice, stream));
+    return reinterpret_cast<const uint32_t*>(x0.ptr);
   }
 
-  static int splits_for(int64_t k) { return (int)std::min<int64_t>(128, std::max<int64_t>(1, k / 2048)); }
-
-  // Forward on x0 (already in this->x0 or given), batch n; logits into out [n][8].
-  void forward(const __nv_bfloat16* in, int64_t n)
+  // Forward on `in` (batch n); with targets [n][6] also the loss, dL/dout and the dense layers'
+  // data gradients.  Logits into out [n][8].
+  void forward(const uint32_t* in, int64_t n, const float* target)
   {
     using L = cnn::WeightLayout;
     using P = cnn::ParamLayout;
-    const __nv_bfloat16* acts_in[4] = {in, a1.ptr, a2.ptr, a3.ptr};
-    __nv_bfloat16* acts_out[4] = {a1.ptr, a2.ptr, a3.ptr, a4.ptr};
-    const int woff[4] = {L::c1, L::c2, L::c3, L::c4};
-    const int boff[4] = {P::b1, P::b2, P::b3, P::b4};
-    for (int l = 0; l < 4; ++l)
-    {
-      const int si = cnn::side_of(l), so = cnn::side_of(l + 1), ci = l == 0 ? 2 : 32;
-      cnn::ConvFwdOp op;
-      op.in = acts_in[l];
-      op.w = wb.ptr + woff[l];
-      op.bias = params.ptr + boff[l];
-      op.out = acts_out[l];
-      op.M = n * so * so;
-      op.N = 32;
-      op.splits = 1;
-      op.kreal = 9 * ci;
-      op.kpad = l == 0 ? cnn::kC1K : 288;
-      op.K = op.kpad;
-      op.si = si;
-      op.so = so;
-      op.ci = ci;
-      gemm(op, op.M, 32);
-    }
-    cnn::LinearFwdOp f1{a4.ptr, wb.ptr + L::f1, params.ptr + P::b5, a5.ptr, nullptr, n, cnn::kHidden, 1, 128, 0};
-    gemm(f1, n, cnn::kHidden);
-    cnn::LinearFwdOp f2{a5.ptr, wb.ptr + L::f2, params.ptr + P::b6, nullptr, out.ptr, n, cnn::kOut, 1, cnn::kHidden,
-                        cnn::kOutPad};
-    gemm(f2, n, cnn::kOutPad);
+    cnn::k_conv1_fwd<<<tile_grid(n * 256, 8), cnn::kTrainThreads, 0, stream>>>(in, wb.ptr, params.ptr, a1.ptr, n);
+    check("k_conv1_fwd");
+    cnn::k_conv_fwd<8><<<tile_grid(n * 64, 4), cnn::kTrainThreads, 0, stream>>>(a1.ptr, wb.ptr + L::c2, params.ptr + P::b2,
+                                                                               a2.ptr, n);
+    cnn::k_conv_fwd<4><<<tile_grid(n * 16, 4), cnn::kTrainThreads, 0, stream>>>(a2.ptr, wb.ptr + L::c3, params.ptr + P::b3,
+                                                                               a3.ptr, n);
+    cnn::k_conv_fwd<2><<<tile_grid(n * 4, 4), cnn::kTrainThreads, 0, stream>>>(a3.ptr, wb.ptr + L::c4, params.ptr + P::b4,
+                                                                              a4.ptr, n);
+    launches += 2;
+    check("k_conv_fwd");
+    const unsigned grid = (unsigned)std::min<int64_t>((n + 15) / 16, (int64_t)sms * 2);
+    cnn::k_mlp<<<grid, cnn::kTrainThreads, sizeof(cnn::MlpSmem), stream>>>(a4.ptr, wb.ptr, params.ptr, target, n, a5.ptr,
+                                                                          out.ptr, dout.ptr, row_loss.ptr, d5.ptr, d4.ptr);
+    check("k_mlp");
   }
 
-  void reduce_into(int splits, int rows, int cols, int keep, float* dst, int ld)
-  {
-    const int total = rows * keep;
-    cnn::k_reduce_splits<<<(total + 255) / 256, 256, 0, stream>>>(part.ptr, splits, rows, cols, keep, dst, ld);
-    check("k_reduce_splits");
-  }
-
-  void bias_grad(const __nv_bfloat16* dz, int64_t rows, int ld, int ncol, float* db)
-  {
-    cnn::k_bias_grad<<<ncol, 256, 0, stream>>>(dz, rows, ld, ncol, db);
-    check("k_bias_grad");
-  }
-
-  // Backward after forward(in, n) with targets [n][6]; gradients into grads (param layout).
-  void backward(const __nv_bfloat16* in, const float* target, int64_t n)
+  // Backward after forward(in, n, target); gradients into grads (param layout).
+  void backward(const uint32_t* in, int64_t n)
   {
     using L = cnn::WeightLayout;
-    using P = cnn::ParamLayout;
-    cnn::k_loss_grad<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(out.ptr, target, n, dout.ptr, row_loss.ptr);
-    check("k_loss_grad");
-    // f2
-    {
-      const int S = splits_for(n);
-      cnn::LinearBwdWeightOp op{dout.ptr, a5.ptr, part.ptr, cnn::kOut, cnn::kHidden, S, n, cnn::kOutPad};
-      gemm(op, cnn::kOut, cnn::kHidden);
-      reduce_into(S, cnn::kOut, cnn::kHidden, cnn::kHidden, grads.ptr + P::w6, cnn::kHidden);
-      bias_grad(dout.ptr, n, cnn::kOutPad, cnn::kOut, grads.ptr + P::b6);
-      cnn::LinearBwdDataOp dop{dout.ptr, wb.ptr + L::f2, a5.ptr, d5.ptr, n, cnn::kHidden, 1, cnn::kOut, cnn::kOutPad};
-      gemm(dop, n, cnn::kHidden);
-    }
-    // f1
-    {
-      const int S = splits_for(n);
-      cnn::LinearBwdWeightOp op{d5.ptr, a4.ptr, part.ptr, cnn::kHidden, 128, S, n, cnn::kHidden};
-      gemm(op, cnn::kHidden, 128);
-      reduce_into(S, cnn::kHidden, 128, 128, grads.ptr + P::w5, 128);
-      bias_grad(d5.ptr, n, cnn::kHidden, cnn::kHidden, grads.ptr + P::b5);
-      cnn::LinearBwdDataOp dop{d5.ptr, wb.ptr + L::f1, a4.ptr, d4.ptr, n, 128, 1, cnn::kHidden, cnn::kHidden};
-      gemm(dop, n, 128);
-    }
-    // conv4 .. conv1
-    const __nv_bfloat16* acts_in[4] = {in, a1.ptr, a2.ptr, a3.ptr};
-    __nv_bfloat16* dz_out[4] = {d1.ptr, d2.ptr, d3.ptr, d4.ptr};
-    const int woff[4] = {L::c1, L::c2, L::c3, L::c4};
-    const int wpo[4] = {P::w1, P::w2, P::w3, P::w4};
-    const int bpo[4] = {P::b1, P::b2, P::b3, P::b4};
-    for (int l = 3; l >= 0; --l)
-    {
-      const int si = cnn::side_of(l), so = cnn::side_of(l + 1), ci = l == 0 ? 2 : 32;
-      const int kreal = 9 * ci, kpad = l == 0 ? cnn::kC1K : 288;
-      const int64_t K = n * so * so;
-      const int S = splits_for(K);
-      cnn::ConvBwdWeightOp wop{dz_out[l], acts_in[l], part.ptr, 32, kpad, S, K, si, so, ci, 32, kreal, kpad};
-      gemm(wop, 32, kpad);
-      reduce_into(S, 32, kpad, kreal, grads.ptr + wpo[l], kreal);
-      bias_grad(dz_out[l], K, 32, 32, grads.ptr + bpo[l]);
-      if (l > 0)
-      {
-        cnn::ConvBwdDataOp dop{dz_out[l], wb.ptr + woff[l], acts_in[l], dz_out[l - 1], n * si * si, ci, 1, 9 * 32,
-                               si, so, ci, 32, kpad};
-        gemm(dop, n * si * si, ci);
-      }
-    }
+    cnn::PartLayout parts;
+    const auto split = [&](int64_t groups, int most) { return (int)std::min<int64_t>(groups, most); };
+    parts.parts[0] = split(n, cnn::kMaxParts);
+    parts.parts[1] = split(n, cnn::kMaxParts);
+    parts.parts[2] = split((n + 3) / 4, cnn::kMaxParts);
+    parts.parts[3] = split((n + 15) / 16, cnn::kMaxParts);
+    parts.parts[4] = split((n + cnn::kMlpStage - 1) / cnn::kMlpStage, cnn::kMlpParts);
+    float* conv = part.ptr + cnn::kPartConv;
+    constexpr size_t layer = (size_t)cnn::kMaxParts * cnn::kConvPart;
+    cnn::k_mlp_wgrad<<<parts.parts[4], cnn::kTrainThreads, sizeof(cnn::MlpWgradSmem), stream>>>(
+        dout.ptr, d5.ptr, a5.ptr, a4.ptr, part.ptr + cnn::kPartMlp, n);
+    check("k_mlp_wgrad");
+    cnn::k_conv_wgrad<2><<<parts.parts[3], cnn::kWgradThreads, 2 * sizeof(cnn::WgradStage<2>), stream>>>(
+        d4.ptr, a3.ptr, conv + 2 * layer, n);
+    cnn::k_conv_dgrad<2><<<tile_grid(n * 4, 4), cnn::kTrainThreads, 0, stream>>>(d4.ptr, wb.ptr + L::c4, a3.ptr, d3.ptr, n);
+    cnn::k_conv_wgrad<4><<<parts.parts[2], cnn::kWgradThreads, 2 * sizeof(cnn::WgradStage<4>), stream>>>(
+        d3.ptr, a2.ptr, conv + layer, n);
+    cnn::k_conv_dgrad<4><<<tile_grid(n * 16, 4), cnn::kTrainThreads, 0, stream>>>(d3.ptr, wb.ptr + L::c3, a2.ptr, d2.ptr, n);
+    cnn::k_conv_wgrad<8><<<parts.parts[1], cnn::kWgradThreads, 2 * sizeof(cnn::WgradStage<8>), stream>>>(d2.ptr, a1.ptr,
+                                                                                                       conv, n);
+    cnn::k_conv_dgrad<8><<<tile_grid(n * 64, 4), cnn::kTrainThreads, 0, stream>>>(d2.ptr, wb.ptr + L::c2, a1.ptr, d1.ptr, n);
+    launches += 5;
+    check("k_conv_wgrad / k_conv_dgrad");
+    cnn::k_conv1_wgrad<<<parts.parts[0], cnn::kTrainThreads, 2 * sizeof(cnn::Wgrad1Stage), stream>>>(
+        d1.ptr, in, part.ptr + cnn::kPartConv1, n);
+    check("k_conv1_wgrad");
+    cnn::k_reduce_parts<<<(cnn::ParamLayout::count + 31) / 32, 256, 0, stream>>>(part.ptr, parts, grads.ptr);
+    check("k_reduce_parts");
   }
 
   float loss(int64_t n)
@@ -3090,7 +3048,17 @@ int dic_cnn_create(int32_t device, dic_cnn** out)
     c->adam_m.ensure(np);
     c->adam_v.ensure(np);
     c->wb.ensure(cnn::WeightLayout::count);
-    c->part.ensure((size_t)128 * cnn::kHidden * 128);
+    c->part.ensure(cnn::kPartFloats);
+    DIC_CUDA(cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device));
+    const auto opt_in = [](const void* k, size_t bytes) {
+      DIC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    };
+    opt_in((const void*)cnn::k_mlp, sizeof(cnn::MlpSmem));
+    opt_in((const void*)cnn::k_mlp_wgrad, sizeof(cnn::MlpWgradSmem));
+    opt_in((const void*)cnn::k_conv_wgrad<8>, 2 * sizeof(cnn::WgradStage<8>));
+    opt_in((const void*)cnn::k_conv_wgrad<4>, 2 * sizeof(cnn::WgradStage<4>));
+    opt_in((const void*)cnn::k_conv_wgrad<2>, 2 * sizeof(cnn::WgradStage<2>));
+    opt_in((const void*)cnn::k_conv1_wgrad, 2 * sizeof(cnn::Wgrad1Stage));
     DIC_CUDA(cudaMemsetAsync(c->params.ptr, 0, sizeof(float) * np, c->stream));
     DIC_CUDA(cudaMemsetAsync(c->grads.ptr, 0, sizeof(float) * np, c->stream));
     DIC_CUDA(cudaMemsetAsync(c->adam_m.ptr, 0, sizeof(float) * np, c->stream));
@@ -3189,7 +3157,7 @@ int dic_cnn_forward(dic_cnn* c, const void* d_x0, int64_t n, float* d_out)
     if (!d_x0 || !d_out || n < 0) throw DicError{DIC_ERR_ARGUMENT, "cnn_forward: bad arguments"};
     if (n == 0) return;
     c->ensure_batch(n);
-    c->forward(static_cast<const __nv_bfloat16*>(d_x0), n);
+    c->forward(c->pixels(d_x0, n), n, nullptr);
     DIC_CUDA(cudaMemcpyAsync(d_out, c->out.ptr, sizeof(float) * n * cnn::kOutPad, cudaMemcpyDeviceToDevice, c->stream));
     DIC_CUDA(cudaStreamSynchronize(c->stream));
   });
@@ -3200,9 +3168,9 @@ int dic_cnn_gradient(dic_cnn* c, const void* d_x0, const float* d_target, int64_
   return cnn_guarded(c, [&] {
     if (!d_x0 || !d_target || !d_grad || n <= 0) throw DicError{DIC_ERR_ARGUMENT, "cnn_gradient: bad arguments"};
     c->ensure_batch(n);
-    const __nv_bfloat16* in = static_cast<const __nv_bfloat16*>(d_x0);
-    c->forward(in, n);
-    c->backward(in, d_target, n);
+    const uint32_t* in = c->pixels(d_x0, n);
+    c->forward(in, n, d_target);
+    c->backward(in, n);
     DIC_CUDA(cudaMemcpyAsync(d_grad, c->grads.ptr, sizeof(float) * cnn::ParamLayout::count,
                              cudaMemcpyDeviceToDevice, c->stream));
     const float l = c->loss(n);
@@ -3215,9 +3183,9 @@ int dic_cnn_train_step(dic_cnn* c, const void* d_x0, const float* d_target, int6
   return cnn_guarded(c, [&] {
     if (!d_x0 || !d_target || n <= 0 || !(lr > 0.f)) throw DicError{DIC_ERR_ARGUMENT, "cnn_train_step: bad arguments"};
     c->ensure_batch(n);
-    const __nv_bfloat16* in = static_cast<const __nv_bfloat16*>(d_x0);
-    c->forward(in, n);
-    c->backward(in, d_target, n);
+    const uint32_t* in = c->pixels(d_x0, n);
+    c->forward(in, n, d_target);
+    c->backward(in, n);
     ++c->adam_t;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - std::pow(b1, (float)c->adam_t), c2 = 1.f - std::pow(b2, (float)c->adam_t);
