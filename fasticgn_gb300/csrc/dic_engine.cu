@@ -723,8 +723,14 @@ struct dic_engine
   }
   DevBuf<unsigned long long> icgn_next;   // work counter of the persistent single-queue launch
 
+  // Subsets of at most 16 columns take the form with two POIs per warp (k_icgn_px_half): one
+  // POI leaves half the lanes idle.
+  static int px_per_warp(int rx) { return 2 * rx + 1 <= kHalf ? 2 : 1; }
   // k_icgn_px: dynamic shared memory of one CTA (the warps' windows plus alignment room)
-  static size_t px_smem(int warps, int rx, int ry) { return 128 + (size_t)warps * px_window_bytes(rx, ry); }
+  static size_t px_smem(int warps, int rx, int ry)
+  {
+    return 128 + (size_t)warps * px_per_warp(rx) * px_window_bytes(rx, ry);
+  }
   // the shared-memory opt-in of the three k_icgn_px widths (per engine, so per device): the
   // device's per-block maximum, set once outside any capture
   bool px_attr_set = false;
@@ -744,6 +750,12 @@ struct dic_engine
     opt_in((const void*)k_icgn_px<2, 1>);
     opt_in((const void*)k_icgn_px<4, 1>);
     opt_in((const void*)k_icgn_px<8, 1>);
+    opt_in((const void*)k_icgn_px_half<2, 2>);
+    opt_in((const void*)k_icgn_px_half<4, 2>);
+    opt_in((const void*)k_icgn_px_half<8, 2>);
+    opt_in((const void*)k_icgn_px_half<2, 1>);
+    opt_in((const void*)k_icgn_px_half<4, 1>);
+    opt_in((const void*)k_icgn_px_half<8, 1>);
     opt_in((const void*)k_icgn_batch_px<2, 2>);
     opt_in((const void*)k_icgn_batch_px<4, 2>);
     opt_in((const void*)k_icgn_batch_px<8, 2>);
@@ -764,13 +776,16 @@ struct dic_engine
     px_attr_set = true;
   }
   template <int W>
-  static int max_ctas_px(size_t smem)
+  static int max_ctas_px(size_t smem, int rx)
   {
+    const bool two = px_per_warp(rx) == 2;
     int b = 0;
     if (smem)
-      DIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_icgn_px<W, 2>, W * 32, smem));
+      DIC_CUDA(two ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_icgn_px_half<W, 2>, W * 32, smem)
+                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_icgn_px<W, 2>, W * 32, smem));
     else
-      DIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_icgn_px<W, 0>, W * 32, smem));
+      DIC_CUDA(two ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_icgn_px_half<W, 0>, W * 32, smem)
+                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_icgn_px<W, 0>, W * 32, smem));
     return b;
   }
   int occupancy_batch_px(int warps, size_t smem)
@@ -796,7 +811,7 @@ struct dic_engine
     if (o.warps == warps && o.rx == rx && o.ry == ry) return o.ctas;
     px_attributes();
     const size_t smem = staged ? px_smem(warps, rx, ry) : 0;
-    const int b = warps == 2 ? max_ctas_px<2>(smem) : warps == 8 ? max_ctas_px<8>(smem) : max_ctas_px<4>(smem);
+    const int b = warps == 2 ? max_ctas_px<2>(smem, rx) : warps == 8 ? max_ctas_px<8>(smem, rx) : max_ctas_px<4>(smem, rx);
     if (b < 1) throw DicError{DIC_ERR_ARGUMENT, "IC-GN pixel windows of this subset radius do not fit in shared memory"};
     o = PxOcc{warps, staged ? 1 : 0, rx, ry, b};
     return b;
@@ -842,7 +857,8 @@ struct dic_engine
     px_attributes();
     const size_t smem = sh.tile ? px_smem(warps, p.rx, p.ry) : 0;
     const int ctas = sh.ctas_per_sm > 0 ? sh.ctas_per_sm : occupancy_px(warps, sh.tile != 0, p.rx, p.ry);
-    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)sms * ctas, (p.n + warps - 1) / warps));
+    const int per_cta = warps * px_per_warp(p.rx);
+    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)sms * ctas, (p.n + per_cta - 1) / per_cta));
     const CUtensorMap* m =
         sh.tile == 1 ? tar_map(p.tar, p.w, p.h, px_pitch(p.w), px_window_x(p.rx), px_window_y(p.ry)) : nullptr;
     CUtensorMap none{};
@@ -850,7 +866,14 @@ struct dic_engine
     q.wait_polls = wait_polls;
     q.wait_test = wait_test & 1;
     const int mode = sh.tile ? (m ? 2 : 1) : 0;   // 2: TMA, 1: warp copies, 0: no window
-#define DIC_PX_LAUNCH(W, M) k_icgn_px<W, M><<<grid, W * 32, smem, stream>>>(q, m ? *m : none, icgn_next.ptr, wait_flag())
+#define DIC_PX_LAUNCH(W, M)                                                                                    \
+  do                                                                                                              \
+  {                                                                                                               \
+    if (px_per_warp(p.rx) == 2)                                                                                   \
+      k_icgn_px_half<W, M><<<grid, W * 32, smem, stream>>>(q, m ? *m : none, icgn_next.ptr, wait_flag());         \
+    else                                                                                                          \
+      k_icgn_px<W, M><<<grid, W * 32, smem, stream>>>(q, m ? *m : none, icgn_next.ptr, wait_flag());              \
+  } while (0)
 #define DIC_PX_MODES(W)                       \
   do                                          \
   {                                           \

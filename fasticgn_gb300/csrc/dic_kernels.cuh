@@ -1089,14 +1089,15 @@ __device__ __forceinline__ float sample_pixels(const PixelTile& T, const float* 
 // interpolation range and has its support inside the window.  Sample coordinates are
 // px + fmaf(W1, ly, fmaf(W0, lx, W2)) (y likewise), rounded monotone functions of lx and of
 // ly, so their extremes are the subset's corners, computed here with the same expression;
-// lanes 0-3 take one corner each.  Warp-uniform.
+// lanes corner = 0-3 of a group (the warp, or a half of it) take one corner each; the answer is
+// uniform over the group.
 __device__ __forceinline__ bool window_covers(const float (&W)[6], float px, float py, int rx, int ry, float xmax,
-                                              float ymax, const PixelTile& T, int lane)
+                                              float ymax, const PixelTile& T, int corner, unsigned group)
 {
   bool ok = true;
-  if (lane < 4)
+  if (corner < 4)
   {
-    const float flx = (lane & 1) ? (float)rx : (float)-rx, fly = (lane & 2) ? (float)ry : (float)-ry;
+    const float flx = (corner & 1) ? (float)rx : (float)-rx, fly = (corner & 2) ? (float)ry : (float)-ry;
     const float gxp = px + fmaf(W[1], fly, fmaf(W[0], flx, W[2]));
     const float gyp = py + fmaf(W[4], fly, fmaf(W[3], flx, W[5]));
     ok = gxp >= 1.f && gyp >= 1.f && gxp < xmax && gyp < ymax;
@@ -1106,7 +1107,12 @@ __device__ __forceinline__ bool window_covers(const float (&W)[6], float px, flo
       ok = tx >= 0 && ty >= 0 && tx <= T.bx - 4 && ty <= T.by - 4;
     }
   }
-  return __all_sync(kFull, ok);
+  return (__ballot_sync(kFull, !ok) & group) == 0;
+}
+__device__ __forceinline__ bool window_covers(const float (&W)[6], float px, float py, int rx, int ry, float xmax,
+                                              float ymax, const PixelTile& T, int lane)
+{
+  return window_covers(W, px, py, rx, ry, xmax, ymax, T, lane, kFull);
 }
 
 // the pixel at an integer sample (the lattice case of sample_pixels)
@@ -2128,6 +2134,62 @@ __host__ __device__ constexpr size_t px_window_bytes(int rx, int ry)
   return ((size_t)px_window_x(rx) * px_window_y(ry) * sizeof(float) + 127) & ~(size_t)127;
 }
 
+// Origin of POI poi's window; returns whether the block that its warped subset needs fits.
+__device__ __forceinline__ int px_origin(const IcgnParams& P, const dic_poi* poi, int bx, int by, int& ox, int& oy)
+{
+  const int rx = P.rx, ry = P.ry, w = P.w, h = P.h;
+  int fits = 0;
+  const float px = poi->x, py = poi->y, u = poi->u, v = poi->v;
+  const float W0 = 1.f + poi->ux, W1 = poi->uy, W3 = poi->vx, W4 = 1.f + poi->vy;
+  // only POIs the solver will sample (the entry test passes a non-negative incoming zncc)
+  if (poi->zncc >= 0.f && isfinite(u) && isfinite(v) && isfinite(W0) && isfinite(W1) && isfinite(W3) &&
+      isfinite(W4) && fabsf(u) < w && fabsf(v) < h)
+  {
+    float x0 = 3.4e38f, x1 = -3.4e38f, y0 = 3.4e38f, y1 = -3.4e38f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+    {
+      const float lx = (k & 1) ? (float)rx : (float)-rx, ly = (k & 2) ? (float)ry : (float)-ry;
+      const float gx = px + (W0 * lx + W1 * ly + u), gy = py + (W3 * lx + W4 * ly + v);
+      x0 = fminf(x0, gx); x1 = fmaxf(x1, gx);
+      y0 = fminf(y0, gy); y1 = fmaxf(y1, gy);
+    }
+    if (x0 > -1e6f && x1 < 1e6f && y0 > -1e6f && y1 < 1e6f)
+    {
+      const int ax = (int)floorf(x0) - 1 - kPxMargin, ay = (int)floorf(y0) - 1 - kPxMargin;
+      const int ex = (int)floorf(x1) + 2 + kPxMargin, ey = (int)floorf(y1) + 2 + kPxMargin;
+      ox = ax & ~3;   // floor to a multiple of 4 (two's complement)
+      oy = ay;
+      fits = ex - ox < bx && ey - oy < by;
+    }
+  }
+  return fits;
+}
+// The window by plain loads: columns first, first + lanes, ...
+__device__ __forceinline__ void px_copy(const IcgnParams& P, int ox, int oy, int bx, int by, int win_f, int first, int lanes)
+{
+  const int w = P.w, h = P.h;
+  // eight rows' loads in flight before their stores; pixels outside the image as zero
+  for (int c = first; c < bx; c += lanes)
+  {
+    const int gx = ox + c;
+    const bool xin = gx >= 0 && gx < w;
+    for (int r0 = 0; r0 < by; r0 += 8)
+    {
+      float v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+      {
+        const int gy = oy + r0 + j;
+        v[j] = (xin && r0 + j < by && gy >= 0 && gy < h) ? __ldg(P.tar + ((size_t)gy * px_pitch(w) + gx)) : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (r0 + j < by) px_smem[win_f + (r0 + j) * bx + c] = v[j];
+    }
+  }
+}
+
 // Stages POI i's window for the calling warp (px_smem[win_f...], shared address win) and fills T.
 // kMode 2: one TMA copy (map, the warp's mbarrier bar and its phase parity); 1: warp copies;
 // 0: nothing staged (T.bx = 0, every sample from the global plane).  A compile-time mode keeps
@@ -2145,36 +2207,11 @@ __device__ __forceinline__ bool px_stage(const IcgnParams& P, int64_t i, int lan
                                          PixelTile& T, int cls = 0, int* verdict = nullptr, int pair_bar = 0)
 {
   constexpr int mode = kMode;
-  const int rx = P.rx, ry = P.ry, w = P.w, h = P.h;
-  const int bx = px_window_x(rx), by = px_window_y(ry);
+  const int bx = px_window_x(P.rx), by = px_window_y(P.ry);
   int ox = 0, oy = 0, fits = 0;
   if (lane == 0 && mode != 0)
   {
-    const dic_poi* poi = P.pois + i;
-    const float px = poi->x, py = poi->y, u = poi->u, v = poi->v;
-    const float W0 = 1.f + poi->ux, W1 = poi->uy, W3 = poi->vx, W4 = 1.f + poi->vy;
-    // only POIs the solver will sample (the entry test passes a non-negative incoming zncc)
-    if (poi->zncc >= 0.f && isfinite(u) && isfinite(v) && isfinite(W0) && isfinite(W1) && isfinite(W3) &&
-        isfinite(W4) && fabsf(u) < w && fabsf(v) < h)
-    {
-      float x0 = 3.4e38f, x1 = -3.4e38f, y0 = 3.4e38f, y1 = -3.4e38f;
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-      {
-        const float lx = (k & 1) ? (float)rx : (float)-rx, ly = (k & 2) ? (float)ry : (float)-ry;
-        const float gx = px + (W0 * lx + W1 * ly + u), gy = py + (W3 * lx + W4 * ly + v);
-        x0 = fminf(x0, gx); x1 = fmaxf(x1, gx);
-        y0 = fminf(y0, gy); y1 = fmaxf(y1, gy);
-      }
-      if (x0 > -1e6f && x1 < 1e6f && y0 > -1e6f && y1 < 1e6f)
-      {
-        const int ax = (int)floorf(x0) - 1 - kPxMargin, ay = (int)floorf(y0) - 1 - kPxMargin;
-        const int ex = (int)floorf(x1) + 2 + kPxMargin, ey = (int)floorf(y1) + 2 + kPxMargin;
-        ox = ax & ~3;   // floor to a multiple of 4 (two's complement)
-        oy = ay;
-        fits = ex - ox < bx && ey - oy < by;
-      }
-    }
+    fits = px_origin(P, P.pois + i, bx, by, ox, oy);
     if (fits)
     {
       fence_proxy_async_smem();   // this warp's reads of the previous window come first
@@ -2217,26 +2254,7 @@ __device__ __forceinline__ bool px_stage(const IcgnParams& P, int64_t i, int lan
   }
   else
   {
-    // rows of the window by the whole warp, eight rows' loads in flight before their stores;
-    // pixels outside the image as zero
-    for (int c = lane + 32 * cls; c < bx; c += 32 * kPoiWarps)
-    {
-      const int gx = ox + c;
-      const bool xin = gx >= 0 && gx < w;
-      for (int r0 = 0; r0 < by; r0 += 8)
-      {
-        float v[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-        {
-          const int gy = oy + r0 + j;
-          v[j] = (xin && r0 + j < by && gy >= 0 && gy < h) ? __ldg(P.tar + ((size_t)gy * px_pitch(w) + gx)) : 0.f;
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if (r0 + j < by) px_smem[win_f + (r0 + j) * bx + c] = v[j];
-      }
-    }
+    px_copy(P, ox, oy, bx, by, win_f, lane + 32 * cls, 32 * kPoiWarps);
     if constexpr (kPoiWarps == 2)
       pair_sync(pair_bar);
     else
@@ -2286,6 +2304,34 @@ constexpr int kRefFloats = sizeof(PoiRef) / sizeof(float);
 constexpr int kRefNorm = offsetof(PoiRef, ref_norm) / 4, kRefNormSq = offsetof(PoiRef, ref_norm_sq) / 4,
               kRefSumRc = offsetof(PoiRef, sum_rc) / 4, kRefS = offsetof(PoiRef, S) / 4, kRefG = offsetof(PoiRef, G) / 4,
               kRefInvH = offsetof(PoiRef, inv_h) / 4;
+
+// The record of a POI whose iteration ended without a rejection.
+__device__ __forceinline__ void icgn_store(dic_poi* poi, const float* ref, const float (&W)[6], float s, float tnorm_sq,
+                                           float tc_rc, float conv, int it, const IcgnParams& P)
+{
+  const float ref_norm = ref[kRefNorm];
+  const float esq = s * s * tnorm_sq - 2.f * s * tc_rc + ref[kRefNormSq];
+  const float znssd = esq / (ref_norm * ref_norm);
+  float u = W[2], v = W[5];
+  float zncc = 0.5f * (2.f - znssd);
+  if (conv >= P.conv && (float)it >= P.max_iter) zncc = -4.f;
+  // The incoming guess is re-read here (the record is still unmodified) rather than kept
+  // live across the iteration loop.
+  const float u_init = poi->u, v_init = poi->v;
+  if (isnan(zncc) || isnan(u) || isnan(v))
+  {
+    u = u_init;
+    v = v_init;
+    zncc = -5.f;
+  }
+  poi->u = u; poi->ux = W[0] - 1.f; poi->uy = W[1];
+  poi->v = v; poi->vx = W[3]; poi->vy = W[4] - 1.f;
+  poi->u0 = u_init;
+  poi->v0 = v_init;
+  poi->zncc = zncc;
+  poi->iteration = (float)it;
+  poi->convergence = conv;
+}
 
 // One POI (queue index i) on the calling warp under pixel sampling, column walk: icgn_solve's
 // rules, codes and outputs from the staged window T.  ref: the warp's copy of the POI's record.
@@ -2369,28 +2415,7 @@ __device__ __forceinline__ void icgn_solve_px(const IcgnParams& P, int64_t i, in
   if (P.iter_sum) atomicAdd(P.iter_sum, (unsigned long long)it);
   if (status == -3) { poi->zncc = -3.f; return; }   // src/oc_icgn.cpp:285-289
   if (status == -5) { poi->zncc = -5.f; return; }   // :297-301
-  const float ref_norm = ref[kRefNorm];
-  const float esq = s * s * tnorm_sq - 2.f * s * tc_rc + ref[kRefNormSq];
-  const float znssd = esq / (ref_norm * ref_norm);
-  float u = W[2], v = W[5];
-  float zncc = 0.5f * (2.f - znssd);
-  if (conv >= P.conv && (float)it >= P.max_iter) zncc = -4.f;
-  // The incoming guess is re-read here (the record is still unmodified) rather than kept
-  // live across the iteration loop.
-  const float u_init = poi->u, v_init = poi->v;
-  if (isnan(zncc) || isnan(u) || isnan(v))
-  {
-    u = u_init;
-    v = v_init;
-    zncc = -5.f;
-  }
-  poi->u = u; poi->ux = W[0] - 1.f; poi->uy = W[1];
-  poi->v = v; poi->vx = W[3]; poi->vy = W[4] - 1.f;
-  poi->u0 = u_init;
-  poi->v0 = v_init;
-  poi->zncc = zncc;
-  poi->iteration = (float)it;
-  poi->convergence = conv;
+  icgn_store(poi, ref, W, s, tnorm_sq, tc_rc, conv, it, P);
 }
 
 // The POI's reference record on its way to the warp's copy: two floats on lanes 0-27, loaded
@@ -2434,6 +2459,235 @@ __global__ void __launch_bounds__(kWarps * 32, px_min_blocks(kWarps))
     ref_store(refs[warp], rv, lane);
     icgn_solve_px(P, i, lane, T, refs[warp]);
     __syncwarp();   // every lane's reads of this window before the next copy overwrites it
+  }
+}
+
+// --------------------------------------------------------------------------------------
+// Two POIs per warp, for subsets of at most 16 columns (radius <= 7): lanes 0-15 solve one,
+// lanes 16-31 the next of the queue, in lockstep.  With one POI such a subset leaves half the
+// warp idle (15 of 32 lanes at radius 7), so the same instructions solve twice the POIs; a half
+// that converges first waits for the other (neighbours on the grid rarely differ by more than
+// an iteration).  A half's butterfly over 16 lanes pairs lanes as the 32-lane one does once it
+// has added the idle half's zeros: the same bits as icgn_solve_px.  171 024 POIs at radius 7
+// (1036x186, step 1): IC-GN 1.23 -> 0.69 ms.
+// --------------------------------------------------------------------------------------
+constexpr int kHalf = 16;
+// reduce_sums over the calling half (h: lane in it): the value v of {B0..B5, A1, A2} is left on
+// lanes 2 v, 2 v + 1
+__device__ __forceinline__ float reduce_sums_half(const ColumnSums& c, float flx, int h, float& A0, float& A1, float& A2)
+{
+  const float v[8] = {c.B0, flx * c.B0, c.B2, c.B3, flx * c.B3, c.B5, c.A1, c.A2};
+  const bool b3 = h & 8, b2 = h & 4, b1 = h & 2;
+  float x[4], y[2];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) x[j] = (b3 ? v[j + 4] : v[j]) + __shfl_xor_sync(kFull, b3 ? v[j] : v[j + 4], 8);
+#pragma unroll
+  for (int j = 0; j < 2; ++j) y[j] = (b2 ? x[j + 2] : x[j]) + __shfl_xor_sync(kFull, b2 ? x[j] : x[j + 2], 4);
+  float z = (b1 ? y[1] : y[0]) + __shfl_xor_sync(kFull, b1 ? y[0] : y[1], 2);
+  z += __shfl_xor_sync(kFull, z, 1);
+  A0 = c.A0;
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) A0 += __shfl_xor_sync(kFull, A0, o);
+  A1 = __shfl_sync(kFull, z, 12, kHalf);
+  A2 = __shfl_sync(kFull, z, 14, kHalf);
+  return z;
+}
+
+// The two halves' POIs (live: this half has one, queue index i), icgn_solve_px's rules and
+// outputs.  T, ref: the half's window and record.
+__device__ __forceinline__ void icgn_solve_px_half(const IcgnParams& P, int64_t i, bool live, int lane,
+                                                   const PixelTile& T, const float* ref)
+{
+  const int h16 = lane & (kHalf - 1);
+  const unsigned half = lane < kHalf ? 0x0000ffffu : 0xffff0000u;
+  const int w = P.w, h = P.h, rx = P.rx, ry = P.ry;
+  dic_poi* poi = P.pois + i;
+  float px = 0.f, py = 0.f, W[6] = {1.f, 0.f, 0.f, 0.f, 1.f, 0.f};
+  bool run = live;
+  if (live)
+  {
+    px = poi->x;
+    py = poi->y;
+    const float u_in = poi->u, v_in = poi->v, zncc_in = poi->zncc;
+    // Entry test (src/oc_icgn.cpp:184-191).
+    if (py - ry < 0 || px - rx < 0 || py + ry > h - 1 || px + rx > w - 1 || fabsf(u_in) >= w || fabsf(v_in) >= h ||
+        zncc_in < 0 || isnan(u_in) || isnan(v_in))
+    {
+      if (h16 == 0) poi->zncc = zncc_in >= 0 ? -3.f : zncc_in;
+      run = false;
+    }
+    W[0] = 1.f + poi->ux;
+    W[1] = poi->uy;
+    W[2] = u_in;
+    W[3] = poi->vx;
+    W[4] = 1.f + poi->vy;
+    W[5] = v_in;
+  }
+  const bool solve = run;
+  const float t0 = ref[0];
+  const int sw = 2 * rx + 1;
+  const float inv_size = 1.f / (float)(sw * (2 * ry + 1));
+  const float rx2 = (float)(rx * rx), ry2 = (float)(ry * ry);
+  const float xmax = (float)(w - 2), ymax = (float)(h - 2);
+  const float flx = (float)(h16 - rx);
+  const float4* ref_col = P.ref_pack + (run ? (size_t)((int)py - ry) * w + (int)px + (h16 - rx) : 0);
+  int it = 0;
+  float conv = 0.f, s = 0.f, tnorm_sq = 0.f, tc_rc = 0.f;
+  int status = 0;  // 0 ok, -3 out of range, -5 NaN coordinate
+  while (__any_sync(kFull, run))
+  {
+    ColumnSums c{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
+    const bool covered = window_covers(W, px, py, rx, ry, xmax, ymax, T, h16, half);
+    const bool lat = on_lattice(W, px, py), col = run && h16 < sw;
+    const unsigned rows = __ballot_sync(kFull, col && covered && !lat);
+    if (col) c = px_column(T, P.tar, ref_col, w, h, px, py, W, flx, t0, ry, covered, lat, rows);
+    __syncwarp();
+    const unsigned bad = __ballot_sync(kFull, c.bad != 0);
+    if (bad)
+    {
+      // Rare path: classify with the CPU's order (src/oc_icgn.cpp:266-301).
+      bool oob = false;
+      if (col && (bad & half))
+      {
+        const float ax = fmaf(W[0], flx, W[2]), ay = fmaf(W[3], flx, W[5]);
+        for (int r = 0; r < 2 * ry + 1; ++r)
+        {
+          const float fly = (float)(r - ry);
+          const float gxp = px + fmaf(W[1], fly, ax), gyp = py + fmaf(W[4], fly, ay);
+          if (gxp < 1.f || gyp < 1.f || gxp >= xmax || gyp >= ymax) oob = true;
+        }
+      }
+      const unsigned out = __ballot_sync(kFull, oob);
+      if (run && (bad & half))
+      {
+        ++it;
+        status = (out & half) ? -3 : -5;
+        run = false;
+      }
+    }
+    float A0, A1, A2;
+    const float b = reduce_sums_half(c, flx, h16, A0, A1, A2);   // B of row h16 / 2
+    const float mean_tau = A0 * inv_size, tn = fmaf(-A0, mean_tau, A1);
+    // A flat target subset has zero norm; the CPU then divides by zero and the POI ends
+    // as NaN (-5).  Rounding can leave a tiny residue here, so force the same outcome.
+    const float tar_norm = tn > 0.f ? sqrtf(tn) : __int_as_float(0x7fc00000);
+    const float sc = ref[kRefNorm] / tar_norm;
+    const int row = h16 < 12 ? h16 >> 1 : 0;
+    const float num = sc * fmaf(-mean_tau, ref[kRefS + row], b) - ref[kRefG + row];
+    float dp_l = 0.f;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) dp_l += ref[kRefInvH + row * 6 + k] * __shfl_sync(kFull, num, 2 * k, kHalf);
+    float dp[6];
+#pragma unroll
+    for (int a = 0; a < 6; ++a) dp[a] = __shfl_sync(kFull, dp_l, 2 * a, kHalf);
+    if (run)
+    {
+      ++it;
+      s = sc;
+      tnorm_sq = tn;
+      tc_rc = fmaf(-mean_tau, ref[kRefSumRc], A2);
+      compose_update(W, dp);
+      conv = sqrtf(dp[0] * dp[0] + dp[1] * dp[1] * rx2 + dp[2] * dp[2] * ry2 + dp[3] * dp[3] + dp[4] * dp[4] * rx2 +
+                   dp[5] * dp[5] * ry2);
+      run = (float)it < P.max_iter && conv >= P.conv;
+    }
+    __syncwarp();
+  }
+
+  if (h16 != 0 || !solve) return;
+  if (P.iter_sum) atomicAdd(P.iter_sum, (unsigned long long)it);
+  if (status == -3) { poi->zncc = -3.f; return; }   // src/oc_icgn.cpp:285-289
+  if (status == -5) { poi->zncc = -5.f; return; }   // :297-301
+  icgn_store(poi, ref, W, s, tnorm_sq, tc_rc, conv, it, P);
+}
+
+// px_stage for the two halves (i: this half's POI, live: it has one): lanes 0 and 16 bound
+// their POIs' windows and issue the copies, each half on its own barrier and window.
+template <int kMode>
+__device__ __forceinline__ bool px_stage_half(const IcgnParams& P, int64_t i, bool live, int lane, int win_f, uint32_t win,
+                                              const CUtensorMap* map, uint32_t bar, uint32_t& parity, int* err, PixelTile& T)
+{
+  const int bx = px_window_x(P.rx), by = px_window_y(P.ry);
+  const int h16 = lane & (kHalf - 1);
+  int ox = 0, oy = 0, fits = 0;
+  if (h16 == 0 && live && kMode != 0)
+  {
+    fits = px_origin(P, P.pois + i, bx, by, ox, oy);
+    if (fits)
+    {
+      fence_proxy_async_smem();   // this half's reads of the previous window come first
+      if (kMode == 2)
+      {
+        mbar_arrive_expect_tx(bar, (uint32_t)(bx * by * sizeof(float)));
+        if (!P.wait_test) tma_load_2d(win, map, ox, oy, bar);
+      }
+    }
+  }
+  __syncwarp();
+  ox = __shfl_sync(kFull, ox, 0, kHalf);
+  oy = __shfl_sync(kFull, oy, 0, kHalf);
+  fits = __shfl_sync(kFull, fits, 0, kHalf);
+  T.s = win_f;
+  T.ox = ox;
+  T.oy = oy;
+  T.bx = fits ? bx : 0;
+  T.by = fits ? by : 0;
+  if (kMode == 2)
+  {
+    bool done = true;
+    if (fits)
+    {
+      done = mbar_wait_bounded(bar, parity, P.wait_polls);
+      parity ^= 1u;
+    }
+    if (!__all_sync(kFull, done))
+    {
+      if (h16 == 0 && fits)
+      {
+        atomicOr(err, 1);
+        mbar_wait_bounded(bar, parity ^ 1u, P.wait_polls);   // the copy in flight, once more
+      }
+      return false;
+    }
+  }
+  else if (fits)
+    px_copy(P, ox, oy, bx, by, win_f, h16, kHalf);
+  __syncwarp();
+  return true;
+}
+
+template <int kWarps, int kMode>
+__global__ void __launch_bounds__(kWarps * 32, px_min_blocks(kWarps))
+    k_icgn_px_half(IcgnParams P, const __grid_constant__ CUtensorMap map, unsigned long long* next, int* err)
+{
+  __shared__ __align__(16) float refs[2 * kWarps][kRefFloats];
+  __shared__ __align__(8) unsigned long long bars[2 * kWarps];
+  const int lane = threadIdx.x & 31, slot = threadIdx.x / kHalf, h16 = lane & (kHalf - 1);
+  if (P.enable && *P.enable == 0) return;
+  uint32_t win = 0;
+  const int win_f = px_window(slot, px_window_bytes(P.rx, P.ry), win);
+  const uint32_t bar = smem_addr(&bars[slot]);
+  if (h16 == 0) mbar_init(bar, 1);
+  __syncwarp();
+  uint32_t parity = 0;
+  for (;;)
+  {
+    unsigned long long t = 0;
+    if (lane == 0) t = atomicAdd(next, 2ull);
+    const int64_t i0 = (int64_t)__shfl_sync(kFull, t, 0);
+    if (!queue_slot_active(P, i0)) return;
+    const int64_t i = i0 + lane / kHalf;
+    const bool live = queue_slot_active(P, i);
+    // the record: 56 floats by 14 lanes of the half
+    float4 rv = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (live && h16 < kRefFloats / 4)
+      rv = __ldg(reinterpret_cast<const float4*>(P.poi_ref + (P.slot ? P.slot[i] : i)) + h16);
+    PixelTile T;
+    if (!px_stage_half<kMode>(P, i, live, lane, win_f, win, &map, bar, parity, err, T)) return;
+    if (h16 < kRefFloats / 4) reinterpret_cast<float4*>(refs[slot])[h16] = rv;
+    __syncwarp();
+    icgn_solve_px_half(P, i, live, lane, T, refs[slot]);
+    __syncwarp();   // both halves' reads of the windows before the next copies overwrite them
   }
 }
 

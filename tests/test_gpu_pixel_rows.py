@@ -38,3 +38,27 @@ def test_row_loops_equal_the_general_loop(dic, radius, width):
         np.testing.assert_array_equal(q.view(np.uint8), got[0].view(np.uint8))
     if radius >= 7:
         assert (got[0]["zncc"] >= 0).mean() > 0.2
+
+
+@pytest.mark.parametrize("radius,drop", [(1, 0), (2, 1), (5, 0), (7, 0), (7, 1)])
+def test_two_pois_per_warp_equal_one(dic, radius, drop):
+    """Subsets of at most 16 columns: two POIs per warp for a queue, one per warp in a batch.  An
+    odd queue leaves its last warp with one; rejected and unconverged POIs share warps with solved
+    ones."""
+    from fasticgn_gb300 import speckle
+    pr = speckle.pair_bumps(seed=400 + radius, width=232, height=200, max_disp=3.0, max_strain=0.03)
+    q = dic.grid_queue(232, 200, radius, 3)
+    q = np.ascontiguousarray(q[:len(q) - (len(q) + drop + 1) % 2])     # odd (drop 0) or even
+    assert len(q) % 2 == 1 - drop
+    rng = np.random.default_rng(radius)
+    far = rng.random(len(q)) < 0.1
+    q["x"][far] += rng.integers(-40, 40, far.sum())                     # some subsets leave the image
+    q["zncc"][rng.random(len(q)) < 0.05] = -3
+    want, got = q.copy(), q.copy()
+    with dic.Engine(radius) as e:
+        e.batch_process([(pr.ref, pr.tar, radius, want)])
+    with dic.Engine(radius) as e:
+        e.set_ref(pr.ref)
+        e.set_tar(pr.tar)
+        e.process_pair(got)
+    np.testing.assert_array_equal(got.view(np.uint8), want.view(np.uint8))
