@@ -340,11 +340,42 @@ __device__ __forceinline__ void solve6_column(const float (&a)[6][6], const int 
 // 21 Hessian entries from them once; S and G likewise (S_1 = lx * sum gx, ...).  The
 // target-side sums of k_icgn use the same forms, which keeps the exact self-match.
 // --------------------------------------------------------------------------------------
-// Sums of one POI's reference subset, butterfly-reduced so every lane holds them.
+// Sums of one POI's reference subset.  The 32 values in lane order -- H's lower triangle (0-20),
+// S (21-26), G 0-4 (27-31) -- leave one per lane; the last one of G, nsq and src on every lane.
 struct PoiSums
 {
-  float nsq, src, S[6], G[6], H[21];
+  float v, g5, nsq, src;
 };
+constexpr int kSumS = 21, kSumG = 27;
+
+// The lanes' sums of 32 values m[l] * q[l], value l on lane l: an xor butterfly over 16, 8, 4, 2, 1
+// that halves the values on the way (each lane keeps the half its bit selects), 31 shuffles for
+// 160.  The pairings are warp_sum's, and so are the bits.  kFused (the pair walk): H's entries
+// (3,1), (4,0) and (4,2) enter their first addition unrounded, the others as rounded products, so
+// that the pair walk's records stay those of one butterfly per value as the compiler formed it.
+__host__ __device__ constexpr bool sum_fused(int k) { return k == 7 || k == 10 || k == 12; }
+template <bool kFused>
+__device__ __forceinline__ float warp_sum32(const float (&m)[32], const float (&q)[32], int lane)
+{
+  float v[16];
+  const bool up = lane & 16;
+#pragma unroll
+  for (int k = 0; k < 16; ++k)
+  {
+    const float a = __fmul_rn(m[k], q[k]), b = __fmul_rn(m[k + 16], q[k + 16]);
+    const float got = __shfl_xor_sync(kFull, up ? a : b, 16);
+    v[k] = kFused && sum_fused(k) ? __fmaf_rn(up ? 1.f : m[k], up ? b : q[k], got) : __fadd_rn(up ? b : a, got);
+  }
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1)
+  {
+    const bool hi = lane & o;
+#pragma unroll
+    for (int k = 0; k < o; ++k)
+      v[k] = __fadd_rn(hi ? v[k + o] : v[k], __shfl_xor_sync(kFull, hi ? v[k] : v[k + o], o));
+  }
+  return v[0];
+}
 
 // The sums of one subset column that do not depend on the subset's mean, over the rows
 // ly = -ry..ry in order: the grey sum t, the gradient products' row moments
@@ -388,6 +419,32 @@ struct ColSumsShared
   int stride;
 };
 
+// The lane's column sums (q: gradient products' row moments, s4: S's terms, G: the four terms
+// formed with the mean, lx: the column) as a POI's sums over the warp.  H's lower triangle is
+// row-major over sd = [gx, gx lx, gx ly, gy, gy lx, gy ly]: entry (a, b) is a moment times the
+// column factors of sd_a and sd_b,
+//   (1,1) Q0, (lx,1) lx Q0, (lx,lx) lx^2 Q0, (ly,1) Q1, (ly,lx) lx Q1, (ly,ly) Q2.
+template <bool kFused>
+__device__ __forceinline__ PoiSums reduce_poi_sums(const float (&q)[9], const float (&s4)[4], const float (&G)[4], float lx,
+                                                   float nsq, float src, int lane)
+{
+  const float lx2 = lx * lx;
+  const float m[32] = {1.f, lx, lx2, 1.f, lx, 1.f, 1.f, lx, 1.f, 1.f, lx, lx2, lx, lx, lx2, 1.f,
+                       lx, 1.f, 1.f, lx, 1.f, 1.f, lx, 1.f, 1.f, lx, 1.f, 1.f, lx, 1.f, 1.f, lx};
+  const float v[32] = {q[0], q[0], q[0], q[1], q[1], q[2],                  // (0,0) .. (2,2): xx
+                       q[6], q[6], q[7], q[3],                              // (3,*): xy, yy
+                       q[6], q[6], q[7], q[3], q[3],                        // (4,*)
+                       q[7], q[7], q[8], q[4], q[4], q[5],                  // (5,*)
+                       s4[0], s4[0], s4[1], s4[2], s4[2], s4[3],            // S
+                       G[0], G[0], G[1], G[2], G[2]};                       // G 0-4
+  PoiSums r;
+  r.v = warp_sum32<kFused>(m, v, lane);
+  r.g5 = warp_sum(G[3]);
+  r.nsq = warp_sum(nsq);
+  r.src = warp_sum(src);
+  return r;
+}
+
 // Entry test, mean (written to rec->t0), and the warp-reduced sums of one POI.  Returns false
 // (after writing valid = 0) when the reference subset leaves the image.  `shared`: the POI's
 // column sums as k_poi_prepare32 staged them (column and pair walks); otherwise col_sums forms
@@ -409,12 +466,10 @@ __device__ __forceinline__ bool poi_sums(const float4* __restrict__ ref_pack, in
   const int sw = 2 * rx + 1, size = sw * (2 * ry + 1);
   const int cx = (int)px, cy = (int)py;
   float sum = 0.f;
-  float nsq = 0.f, src = 0.f, S[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, G[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  float H[21];
-#pragma unroll
-  for (int t = 0; t < 21; ++t) H[t] = 0.f;
+  float nsq = 0.f, src = 0.f;
   if (sw <= 32)
   {
+    float Gm[4] = {0.f, 0.f, 0.f, 0.f};
     const float4* col = ref_pack + (size_t)(cy - ry) * w + cx + (lane - rx);
     ColSums cs;
     cs.t = 0.f;
@@ -437,15 +492,10 @@ __device__ __forceinline__ bool poi_sums(const float4* __restrict__ ref_pack, in
     }
     sum = warp_sum(cs.t);
     const float t0 = sum / (float)size;
-    const float Qxx[3] = {cs.q[0], cs.q[1], cs.q[2]}, Qyy[3] = {cs.q[3], cs.q[4], cs.q[5]},
-                Qxy[3] = {cs.q[6], cs.q[7], cs.q[8]};
-    S[0] = cs.s[0];
-    S[2] = cs.s[1];
-    S[3] = cs.s[2];
-    S[5] = cs.s[3];
     if (lane < sw)
     {
       // the sums that depend on the mean, per sample in the IC-GN walk's order
+#pragma unroll 4
       for (int r = 0; r < 2 * ry + 1; ++r)
       {
         const float fly = (float)(r - ry);
@@ -454,35 +504,14 @@ __device__ __forceinline__ bool poi_sums(const float4* __restrict__ ref_pack, in
         nsq = fmaf(rc, rc, nsq);
         src += rc;
         const float grc = __fmul_rn(v.y, rc), hrc = __fmul_rn(v.z, rc);
-        G[0] = __fadd_rn(G[0], grc);
-        G[2] = fmaf(grc, fly, G[2]);
-        G[3] = __fadd_rn(G[3], hrc);
-        G[5] = fmaf(hrc, fly, G[5]);
+        Gm[0] = __fadd_rn(Gm[0], grc);
+        Gm[1] = fmaf(grc, fly, Gm[1]);
+        Gm[2] = __fadd_rn(Gm[2], hrc);
+        Gm[3] = fmaf(hrc, fly, Gm[3]);
       }
     }
-    const float lx = (float)(lane - rx), lx2 = lx * lx;
-    G[1] = lx * G[0];
-    G[4] = lx * G[3];
-    S[1] = lx * S[0];
-    S[4] = lx * S[3];
-    // sd = [gx, gx lx, gx ly, gy, gy lx, gy ly]; H lower triangle, row-major (a >= b).
-    // Factor of sd_a sd_b by (f_a, f_b) with f in {1, lx, ly}:
-    //   (1,1) Q0, (lx,1) lx Q0, (lx,lx) lx^2 Q0, (ly,1) Q1, (ly,lx) lx Q1, (ly,ly) Q2.
-    H[0] = Qxx[0];                                   // (0,0)
-    H[1] = lx * Qxx[0];  H[2] = lx2 * Qxx[0];        // (1,0) (1,1)
-    H[3] = Qxx[1];  H[4] = lx * Qxx[1];  H[5] = Qxx[2];   // (2,0) (2,1) (2,2)
-    H[6] = Qxy[0];  H[7] = lx * Qxy[0];  H[8] = Qxy[1];  H[9] = Qyy[0];                 // (3,*)
-    H[10] = lx * Qxy[0];  H[11] = lx2 * Qxy[0];  H[12] = lx * Qxy[1];                   // (4,0..2)
-    H[13] = lx * Qyy[0];  H[14] = lx2 * Qyy[0];                                          // (4,3) (4,4)
-    H[15] = Qxy[1];  H[16] = lx * Qxy[1];  H[17] = Qxy[2];                               // (5,0..2)
-    H[18] = Qyy[1];  H[19] = lx * Qyy[1];  H[20] = Qyy[2];                               // (5,3..5)
-    if (lane >= sw)
-    {
-#pragma unroll
-      for (int t = 0; t < 21; ++t) H[t] = 0.f;
-#pragma unroll
-      for (int a = 0; a < 6; ++a) { S[a] = 0.f; G[a] = 0.f; }
-    }
+    // (lanes past the subset hold zero sums)
+    out_sums = reduce_poi_sums<false>(cs.q, cs.s, Gm, (float)(lane - rx), nsq, src, lane);
     if (lane == 0) rec->t0 = t0;
   }
   else if (sw <= kPairMaxWidth)
@@ -513,7 +542,7 @@ __device__ __forceinline__ bool poi_sums(const float4* __restrict__ ref_pack, in
     for (int k = 0; k < 2; ++k)
     {
       const int c = pair_column(lane, k);
-      float pn = 0.f, ps = 0.f, pS[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, pG[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      float pn = 0.f, ps = 0.f, pG[4] = {0.f, 0.f, 0.f, 0.f};
       ColSums cs;
       cs.t = 0.f;
 #pragma unroll
@@ -529,9 +558,9 @@ __device__ __forceinline__ bool poi_sums(const float4* __restrict__ ref_pack, in
           ps += rc;
           const float grc = __fmul_rn(v.y, rc), hrc = __fmul_rn(v.z, rc);
           pG[0] = __fadd_rn(pG[0], grc);
-          pG[2] = fmaf(grc, fly, pG[2]);
-          pG[3] = __fadd_rn(pG[3], hrc);
-          pG[5] = fmaf(hrc, fly, pG[5]);
+          pG[1] = fmaf(grc, fly, pG[1]);
+          pG[2] = __fadd_rn(pG[2], hrc);
+          pG[3] = fmaf(hrc, fly, pG[3]);
         };
         if (shared.v)
         {
@@ -539,6 +568,7 @@ __device__ __forceinline__ bool poi_sums(const float4* __restrict__ ref_pack, in
           for (int v = 0; v < 9; ++v) cs.q[v] = shared.v[(1 + v) * shared.stride + c];
 #pragma unroll
           for (int v = 0; v < 4; ++v) cs.s[v] = shared.v[(10 + v) * shared.stride + c];
+#pragma unroll 4
           for (int r = 0; r < 2 * ry + 1; ++r) mean_sums(__ldg(&col[(size_t)r * w]), (float)(r - ry));
         }
         else
@@ -550,107 +580,69 @@ __device__ __forceinline__ bool poi_sums(const float4* __restrict__ ref_pack, in
             col_sums_add(cs, v, fly);
           }
       }
-      pS[0] = cs.s[0];
-      pS[2] = cs.s[1];
-      pS[3] = cs.s[2];
-      pS[5] = cs.s[3];
-      const float Qxx[3] = {cs.q[0], cs.q[1], cs.q[2]}, Qyy[3] = {cs.q[3], cs.q[4], cs.q[5]},
-                  Qxy[3] = {cs.q[6], cs.q[7], cs.q[8]};
-      const float lx = (float)(c - rx), lx2 = lx * lx;
-      pG[1] = lx * pG[0];
-      pG[4] = lx * pG[3];
-      pS[1] = lx * pS[0];
-      pS[4] = lx * pS[3];
-      float pH[21] = {Qxx[0], lx * Qxx[0], lx2 * Qxx[0], Qxx[1], lx * Qxx[1], Qxx[2],
-                      Qxy[0], lx * Qxy[0], Qxy[1], Qyy[0],
-                      lx * Qxy[0], lx2 * Qxy[0], lx * Qxy[1], lx * Qyy[0], lx2 * Qyy[0],
-                      Qxy[1], lx * Qxy[1], Qxy[2], Qyy[1], lx * Qyy[1], Qyy[2]};
-      pn = warp_sum(pn);
-      ps = warp_sum(ps);
-#pragma unroll
-      for (int a = 0; a < 6; ++a) { pS[a] = warp_sum(pS[a]); pG[a] = warp_sum(pG[a]); }
-#pragma unroll
-      for (int t = 0; t < 21; ++t) pH[t] = warp_sum(pH[t]);
+      const PoiSums mine = reduce_poi_sums<true>(cs.q, cs.s, pG, (float)(c - rx), pn, ps, lane);
       if (k == 0)
-      {
-        nsq = pn;
-        src = ps;
-#pragma unroll
-        for (int a = 0; a < 6; ++a) { S[a] = pS[a]; G[a] = pG[a]; }
-#pragma unroll
-        for (int t = 0; t < 21; ++t) H[t] = pH[t];
-      }
+        out_sums = mine;
       else
       {
-        nsq = __fadd_rn(nsq, pn);
-        src = __fadd_rn(src, ps);
-#pragma unroll
-        for (int a = 0; a < 6; ++a) { S[a] = __fadd_rn(S[a], pS[a]); G[a] = __fadd_rn(G[a], pG[a]); }
-#pragma unroll
-        for (int t = 0; t < 21; ++t) H[t] = __fadd_rn(H[t], pH[t]);
+        out_sums.v = __fadd_rn(out_sums.v, mine.v);
+        out_sums.g5 = __fadd_rn(out_sums.g5, mine.g5);
+        out_sums.nsq = __fadd_rn(out_sums.nsq, mine.nsq);
+        out_sums.src = __fadd_rn(out_sums.src, mine.src);
       }
     }
     if (lane == 0) rec->t0 = t0;
-#pragma unroll
-    for (int a = 0; a < 6; ++a) { out_sums.S[a] = S[a]; out_sums.G[a] = G[a]; }
-#pragma unroll
-    for (int t = 0; t < 21; ++t) out_sums.H[t] = H[t];
-    out_sums.nsq = nsq;
-    out_sums.src = src;
-    return true;   // already reduced
   }
   else
   {
+    float v[32], one[32], g5 = 0.f;   // H, S, G 0-4 in PoiSums' order
+#pragma unroll
+    for (int k = 0; k < 32; ++k)
+    {
+      v[k] = 0.f;
+      one[k] = 1.f;
+    }
     DIC_FOR_EACH_SAMPLE(lane, rx, ry, sum += __ldg(&ref_pack[(size_t)(cy + ly) * w + cx + lx].x);)
     sum = warp_sum(sum);
     const float t0 = sum / (float)size;
     DIC_FOR_EACH_SAMPLE(lane, rx, ry,
-      const float4 v = __ldg(&ref_pack[(size_t)(cy + ly) * w + cx + lx]);
-      const float rc = v.x - t0;
+      const float4 x = __ldg(&ref_pack[(size_t)(cy + ly) * w + cx + lx]);
+      const float rc = x.x - t0;
       const float flx = (float)lx, fly = (float)ly;
-      const float sd[6] = {v.y, v.y * flx, v.y * fly, v.z, v.z * flx, v.z * fly};
+      const float sd[6] = {x.y, x.y * flx, x.y * fly, x.z, x.z * flx, x.z * fly};
       nsq = fmaf(rc, rc, nsq);
       src += rc;
       int t = 0;
       _Pragma("unroll")
       for (int a = 0; a < 6; ++a)
       {
-        S[a] += sd[a];
-        G[a] = fmaf(sd[a], rc, G[a]);
+        v[kSumS + a] += sd[a];
+        if (a < 5)
+          v[kSumG + a] = fmaf(sd[a], rc, v[kSumG + a]);
+        else
+          g5 = fmaf(sd[a], rc, g5);
         _Pragma("unroll")
-        for (int b = 0; b <= a; ++b) H[t++] += sd[a] * sd[b];
+        for (int b = 0; b <= a; ++b) v[t++] += sd[a] * sd[b];
       }
     )
+    out_sums.v = warp_sum32<false>(one, v, lane);
+    out_sums.g5 = warp_sum(g5);
+    out_sums.nsq = warp_sum(nsq);
+    out_sums.src = warp_sum(src);
     if (lane == 0) rec->t0 = t0;
   }
-  nsq = warp_sum(nsq);
-  src = warp_sum(src);
-#pragma unroll
-  for (int a = 0; a < 6; ++a) { S[a] = warp_sum(S[a]); G[a] = warp_sum(G[a]); }
-#pragma unroll
-  for (int t = 0; t < 21; ++t) H[t] = warp_sum(H[t]);
-#pragma unroll
-  for (int a = 0; a < 6; ++a) { out_sums.S[a] = S[a]; out_sums.G[a] = G[a]; }
-#pragma unroll
-  for (int t = 0; t < 21; ++t) out_sums.H[t] = H[t];
-  out_sums.nsq = nsq;
-  out_sums.src = src;
   return true;
 }
 
-// S and G (lane c < 6 writes entry c, G centred), the norms and valid (lane 0).
+// S, G (centred), the norms and valid, each from the lane that holds it.
 __device__ __forceinline__ void poi_write_sums(const PoiSums& q, int size, int lane, PoiRef* __restrict__ rec)
 {
   const float m_r = q.src * (1.f / (float)size);
-  if (lane < 6)
-  {
-    float S_l = q.S[0], G_l = q.G[0];
-#pragma unroll
-    for (int a = 1; a < 6; ++a)
-      if (lane == a) { S_l = q.S[a]; G_l = q.G[a]; }
-    rec->S[lane] = S_l;
-    rec->G[lane] = fmaf(-m_r, S_l, G_l);
-  }
+  // lanes 27-31 hold G 0-4 and read S 0-4 from lanes 21-25; lane 26 holds S 5, for G 5
+  const float S_l = __shfl_sync(kFull, q.v, lane >= kSumG ? lane - 6 : lane);
+  if (lane >= kSumS && lane < kSumG) rec->S[lane - kSumS] = q.v;
+  if (lane >= kSumG) rec->G[lane - kSumG] = fmaf(-m_r, S_l, q.v);
+  if (lane == kSumG - 1) rec->G[5] = fmaf(-m_r, S_l, q.g5);
   if (lane == 0)
   {
     const float rn_sq = fmaf(-q.src, m_r, q.nsq);
@@ -671,14 +663,18 @@ __global__ void __launch_bounds__(128) k_poi_prepare(const float4* __restrict__ 
   PoiRef* rec = out + i;
   PoiSums q;
   if (!poi_sums(ref_pack, w, h, pois[i].x, pois[i].y, rx, ry, lane, rec, q)) return;
-  // Every lane holds the same sums (butterfly reductions), so the LU runs uniformly and
-  // lane c < 6 solves and writes column c of the inverse.
+  // Every lane takes the whole matrix from the lanes that hold its entries, so the LU runs
+  // uniformly and lane c < 6 solves and writes column c of the inverse.
   float hf[6][6];
   int t = 0;
 #pragma unroll
   for (int a = 0; a < 6; ++a)
 #pragma unroll
-    for (int b = 0; b <= a; ++b) { hf[a][b] = q.H[t]; hf[b][a] = q.H[t]; ++t; }
+    for (int b = 0; b <= a; ++b)
+    {
+      hf[a][b] = hf[b][a] = __shfl_sync(kFull, q.v, t);
+      ++t;
+    }
   int perm[6];
   lu6(hf, perm);
   if (lane < 6)
@@ -704,13 +700,19 @@ __global__ void __launch_bounds__(128) k_poi_prepare(const float4* __restrict__ 
 // order) and the POIs read them from shared memory; only the sums that depend on a POI's mean
 // (norm, G) are formed per POI.  Any other set of POIs takes the per-POI path.  Same bits
 // either way.
+//
+// Bound by the latency of its row loads and by issue: the 35 warp sums of a POI were a third of
+// its instructions as one butterfly each (warp_sum32 halves the values on the way), which also
+// frees the registers for six CTAs per SM with four rows' loads in flight (three rows at five
+// CTAs 0.46, six rows 0.39 / r 30 0.26 ms).  2048x2048 pair at step 4, r 15: 0.50 -> 0.40 ms;
+// 171 024 POIs at r 7: 0.24 -> 0.18; r 20, 29 000 POIs: 0.166 -> 0.094; r 30: 0.23 -> 0.20.
 // --------------------------------------------------------------------------------------
 constexpr int kPrepPois = 32, kPrepWarps = 4;   // (8 warps per 32 POIs: 0.72 against 0.60 ms at 2048^2)
 constexpr int kPrepCols = 256;   // shared columns per grid row (32 POIs at step <= 7 for r 15, <= 6 for r 30)
 #ifndef DIC_PREP_SHARED_COLUMNS
 #define DIC_PREP_SHARED_COLUMNS 1
 #endif
-__global__ void __launch_bounds__(kPrepWarps * 32) k_poi_prepare32(const float4* __restrict__ ref_pack, int w,
+__global__ void __launch_bounds__(kPrepWarps * 32, 6) k_poi_prepare32(const float4* __restrict__ ref_pack, int w,
                                                                   int h, const dic_poi* __restrict__ pois,
                                                                   int64_t n, int rx, int ry,
                                                                   PoiRef* __restrict__ out)
@@ -796,11 +798,7 @@ __global__ void __launch_bounds__(kPrepWarps * 32) k_poi_prepare32(const float4*
       if (live)
       {
         poi_write_sums(q, size, lane, out + i);
-        if (lane == 0)
-        {
-#pragma unroll
-          for (int t = 0; t < 21; ++t) sh_h[p * 21 + t] = q.H[t];
-        }
+        if (lane < 21) sh_h[p * 21 + lane] = q.v;
       }
     }
     if (lane == 0) sh_live[p] = live ? 1 : 0;
