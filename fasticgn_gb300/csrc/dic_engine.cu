@@ -232,6 +232,45 @@ struct dic_cnn
   }
 };
 
+// FFTCC lengths above 32 with the POIs per CTA of k_fftcc_line (as many as fill the warps of the
+// CTA's lines, 34 -> 8 POIs on 272 of 288 threads, while two CTAs or more share an SM) and
+// whether near ties go to the line-DFT kernel (2 x prime) or to k_fftcc_big.
+#define DIC_FFTCC_LINES(X)                                                                             \
+  X(34, 8, true) X(36, 8, false) X(38, 5, true) X(40, 4, false) X(42, 3, false) X(44, 5, false) X(46, 2, true) \
+  X(48, 2, false) X(50, 3, false) X(52, 3, false) X(54, 1, false) X(56, 1, false) X(58, 1, true) X(60, 1, false) \
+  X(62, 1, true) X(64, 1, false)
+constexpr unsigned kNearCtas = 608;   // CTAs of a second pass at most: near ties are rare
+template <int M, int kPois, bool kPrime>
+void launch_fftcc_line(const FftccParams& p, cudaStream_t st)
+{
+  using F = FftccLine<M, kPois>;
+  k_fftcc_line<M, kPois><<<(unsigned)((p.n + kPois - 1) / kPois), F::kThreads, F::kSmem, st>>>(p);
+  const unsigned second = (unsigned)std::min<int64_t>(p.n, kNearCtas);
+  if constexpr (kPrime)
+    k_fftcc_large<<<second, 256, (size_t)2 * M * (M + 1) * sizeof(float2), st>>>(p, M);
+  else
+    k_fftcc_big<M><<<second, kBigThreads, (size_t)M * (M + 1) * sizeof(float2), st>>>(p);
+}
+template <int M>
+void launch_fftcc2(const FftccParams& p, cudaStream_t st)
+{
+  const unsigned blocks = (unsigned)((p.n + 3) / 4);
+  k_fftcc2<M><<<blocks, 64, 0, st>>>(p);
+  if constexpr (fftcc2_near(M)) k_fftcc2<M, true><<<std::min(blocks, kNearCtas), 64, 0, st>>>(p);
+}
+// whether a length's launch fills a list of near ties (FftccParams::near)
+bool fftcc_near(int m) { return m > 32 || (m >= 8 && m <= 30 && fftcc2_near(m)); }
+// the shared-memory opt-in of every k_fftcc_line form on the current device
+void fftcc_attributes()
+{
+#define DIC_FFTCC_OPT(M, PO, PRIME) \
+  DIC_CUDA(cudaFuncSetAttribute(k_fftcc_line<M, PO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FftccLine<M, PO>::kSmem));
+  DIC_FFTCC_LINES(DIC_FFTCC_OPT)
+#undef DIC_FFTCC_OPT
+  DIC_CUDA(cudaFuncSetAttribute(k_fftcc_large, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(2 * kMaxTwiddleN * (kMaxTwiddleN + 1) * sizeof(float2))));
+}
+
 struct dic_engine
 {
   dic_config cfg{};
@@ -1325,26 +1364,34 @@ struct dic_engine
   }
 
   // ---------------------------------------------------------------- solvers
-  // FFTCC launch for an explicit plane pair and (square) radius.
-  void fftcc_launch(const FftccParams& p, int r, cudaStream_t on = nullptr)
+  // FFTCC launch for an explicit plane pair and (square) radius; p.near / near_n must be set where
+  // fftcc_near(2 r).
+  void fftcc_launch(FftccParams p, int r, cudaStream_t on = nullptr)
   {
     cudaStream_t st = on ? on : stream;
-    const unsigned blocks = (unsigned)((p.n + 3) / 4);
+    if (fftcc_near(2 * r))
+    {
+      DIC_CUDA(cudaMemsetAsync(p.near_n, 0, sizeof(unsigned long long), st));
+      ++launches;   // the second pass
+    }
+    else
+    {
+      p.near = nullptr;
+      p.near_n = nullptr;
+    }
     switch (2 * r)
     {
 #define DIC_FFTCC_CASE2(M) \
-  case M: k_fftcc2<M><<<(unsigned)((p.n + 3) / 4), 64, 0, st>>>(p); break;
+  case M: launch_fftcc2<M>(p, st); break;
       DIC_FFTCC_CASE2(8) DIC_FFTCC_CASE2(10) DIC_FFTCC_CASE2(12) DIC_FFTCC_CASE2(14) DIC_FFTCC_CASE2(16)
       DIC_FFTCC_CASE2(18) DIC_FFTCC_CASE2(20) DIC_FFTCC_CASE2(22) DIC_FFTCC_CASE2(24) DIC_FFTCC_CASE2(26)
       DIC_FFTCC_CASE2(28) DIC_FFTCC_CASE2(30)
 #undef DIC_FFTCC_CASE2
-      case 32: k_fftcc<32><<<blocks, 128, 0, st>>>(p); break;
-#define DIC_FFTCC_BIG(M) \
-  case M: k_fftcc_big<M><<<(unsigned)p.n, 128, (size_t)M * (M + 1) * sizeof(float2), st>>>(p); break;
-      // 2r = 2 x prime (34, 38, 46, 58, 62) stays on the line-DFT kernel below
-      DIC_FFTCC_BIG(36) DIC_FFTCC_BIG(40) DIC_FFTCC_BIG(42) DIC_FFTCC_BIG(44) DIC_FFTCC_BIG(48)
-      DIC_FFTCC_BIG(50) DIC_FFTCC_BIG(52) DIC_FFTCC_BIG(54) DIC_FFTCC_BIG(56) DIC_FFTCC_BIG(60) DIC_FFTCC_BIG(64)
-#undef DIC_FFTCC_BIG
+      case 32: k_fftcc<32><<<(unsigned)((p.n + 3) / 4), 128, 0, st>>>(p); break;
+#define DIC_FFTCC_LINE(M, PO, PRIME) \
+  case M: launch_fftcc_line<M, PO, PRIME>(p, st); break;
+      DIC_FFTCC_LINES(DIC_FFTCC_LINE)
+#undef DIC_FFTCC_LINE
       default:
         if (r < 1 || 2 * r > kMaxTwiddleN)
           throw DicError{DIC_ERR_ARGUMENT, "FFTCC supports subset radius 1..32 on this engine"};
@@ -1352,6 +1399,9 @@ struct dic_engine
     }
     check_launch("k_fftcc");
   }
+  // POIs whose correlation peak the second pass decides, of the engine stream's FFTCC launches
+  DevBuf<int64_t> fft_near;
+  DevBuf<unsigned long long> fft_near_n;
 
   void run_fftcc(dic_poi* d_pois, int64_t n, const int64_t* n_dev = nullptr, const int* enable = nullptr)
   {
@@ -1361,6 +1411,13 @@ struct dic_engine
     FftccParams p{ref_f32.ptr, tar_f32.ptr, d_pois, n, w, h};
     p.n_dev = n_dev;
     p.enable = enable;
+    if (fftcc_near(2 * cfg.subset_radius_x))
+    {
+      fft_near.ensure((size_t)n);
+      fft_near_n.ensure(1);
+      p.near = fft_near.ptr;
+      p.near_n = fft_near_n.ptr;
+    }
     mark(kPhFftcc, 0);
     fftcc_launch(p, cfg.subset_radius_x);
     mark(kPhFftcc, 1);
@@ -1708,6 +1765,8 @@ struct dic_engine
   DevBuf<PoiRef> bpoi;
   DevBuf<BatchJob> bjobs;
   DevBuf<unsigned long long> bnext;
+  DevBuf<int64_t> bnear;                // the jobs' near ties, each in its queue slice, and their counts
+  DevBuf<unsigned long long> bnear_n;
 
   template <typename T>
   void prep_planes(const unsigned char* raw_r, const unsigned char* raw_t, int bw, int bh, JobBufs& J, bool table,
@@ -1797,6 +1856,8 @@ struct dic_engine
     bpoi.ensure((size_t)std::max<int64_t>(b_total, 1));
     bjobs.ensure((size_t)nj);
     bnext.ensure(2 + kMaxPairGroups);
+    bnear.ensure((size_t)std::max<int64_t>(b_total, 1));
+    bnear_n.ensure((size_t)nj);
     counters.ensure(1);
     std::vector<BatchJob> table(nj);
     for (int k = 0; k < nj; ++k)
@@ -1917,6 +1978,8 @@ struct dic_engine
           M.ref_pack.ptr, J.width, J.height, q, J.count, r, r, bpoi.ptr + b_first[k]);
       check_launch("k_poi_prepare32");
       FftccParams fp{M.ref_f32.ptr, M.tar_f32.ptr, q, J.count, J.width, J.height};
+      fp.near = bnear.ptr + b_first[k];
+      fp.near_n = bnear_n.ptr + k;
       fftcc_launch(fp, r, st);
     }
     BatchLaunch col{bjobs.ptr, nj, bq.ptr, bpoi.ptr, 0, b_col_end, bnext.ptr, counters.ptr, b_col_rmax};
@@ -2179,8 +2242,7 @@ int dic_engine_create(const dic_config* config, dic_engine** out)
       e->wait_test = std::atoi(t) & 3;
       if (e->wait_test) e->wait_polls = dic_engine::kTestWaitPolls;
     }
-    DIC_CUDA(cudaFuncSetAttribute(k_fftcc_large, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(2 * kMaxTwiddleN * (kMaxTwiddleN + 1) * sizeof(float2))));
+    fftcc_attributes();
     DIC_CUDA(cudaFuncSetAttribute(cnn::k_proposal_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, cnn::kSmTotal));
     for (int p = 0; p < kPhCount; ++p)
       for (int m = 0; m < dic_engine::kMarks; ++m)
@@ -2248,6 +2310,10 @@ void dic_engine_destroy(dic_engine* e)
   e->bjobs.release();
   e->bmaps.release();
   e->bnext.release();
+  e->bnear.release();
+  e->bnear_n.release();
+  e->fft_near.release();
+  e->fft_near_n.release();
   e->icgn_next.release();
   e->wait_err.release();
   e->tune_q.release();

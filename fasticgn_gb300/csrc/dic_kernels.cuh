@@ -15,6 +15,7 @@
 #include <cstdint>
 #include <cuda.h>            // CUtensorMap (the type only; maps are encoded through the runtime's driver entry point)
 #include <cuda_runtime.h>
+#include <utility>
 
 #include "../../include/dic.h"
 
@@ -3090,7 +3091,76 @@ struct Dft<5>
   }
 };
 
-template <int N, int N1 = first_factor(N)>
+// exp(2 pi i K / N) as compile-time constants (Maclaurin series in double: 2 pi < 6.3, 40 terms
+// leave less than 1e-14)
+constexpr double root_part(double x, bool sine)
+{
+  double term = sine ? x : 1.0, sum = term;
+  for (int k = sine ? 2 : 1; k < 40; k += 2)
+  {
+    term = -term * x * x / (k * (k + 1.0));
+    sum += term;
+  }
+  return sum;
+}
+template <int N, int K>
+struct unit_root
+{
+  static constexpr double kAngle = 6.283185307179586476925 * K / N;
+  static constexpr float re = (float)root_part(kAngle, false), im = (float)root_part(kAngle, true);
+};
+
+// Odd prime lengths above 5 by pairs (used where kDirect is false; kDirect keeps Dft's sums of
+// products in the order that decides near ties of the correlation peak, see FftccParams::near).
+template <int N>
+struct DftPaired
+{
+  // Odd prime length: with A_j = x_j + x_(N-j) and B_j = x_j - x_(N-j), the bins k and N - k are
+  // U +- (V.y, -V.x), U = x_0 + sum A_j cos(2 pi j k / N), V = sum B_j sin(2 pi j k / N): two real
+  // products per term instead of a complex one, and half the terms.  The factors are template
+  // arguments' values, so each is an immediate of its FMA (as constant-bank loads they are kept
+  // in registers: 5 KB of spills at N = 31).
+  static constexpr int H = (N - 1) / 2;
+  template <int K, int... J>
+  __device__ __forceinline__ static void bin(const float2 (&A)[H], const float2 (&B)[H], float2& U, float2& V,
+                                             std::integer_sequence<int, J...>)
+  {
+    ((U.x = fmaf(A[J].x, unit_root<N, (J + 1) * K % N>::re, U.x), U.y = fmaf(A[J].y, unit_root<N, (J + 1) * K % N>::re, U.y),
+      V.x = fmaf(B[J].x, unit_root<N, (J + 1) * K % N>::im, V.x), V.y = fmaf(B[J].y, unit_root<N, (J + 1) * K % N>::im, V.y)),
+     ...);
+  }
+  template <int... K>
+  __device__ __forceinline__ static void bins(float2 x0, const float2 (&A)[H], const float2 (&B)[H], float2 (&out)[N],
+                                              std::integer_sequence<int, K...>)
+  {
+    const auto pair = [&](int k, float2 U, float2 V) {
+      out[k] = make_float2(U.x + V.y, U.y - V.x);
+      out[N - k] = make_float2(U.x - V.y, U.y + V.x);
+    };
+    const auto one = [&](auto k) {
+      constexpr int kk = decltype(k)::value;
+      float2 U = x0, V = make_float2(0.f, 0.f);
+      bin<kk>(A, B, U, V, std::make_integer_sequence<int, H>{});
+      pair(kk, U, V);
+    };
+    (one(std::integral_constant<int, K + 1>{}), ...);
+  }
+  __device__ __forceinline__ static void run(const float2 (&in)[N], float2 (&out)[N])
+  {
+    float2 A[H], B[H];
+    float2 sum = in[0];
+#pragma unroll
+    for (int j = 0; j < H; ++j)
+    {
+      A[j] = cadd(in[j + 1], in[N - 1 - j]);
+      B[j] = csub(in[j + 1], in[N - 1 - j]);
+      sum = cadd(sum, A[j]);
+    }
+    out[0] = sum;
+    bins(in[0], A, B, out, std::make_integer_sequence<int, H>{});
+  }
+};
+template <int N, bool kDirect = false, int N1 = first_factor(N)>
 struct Fft
 {
   static constexpr int N2 = N / N1;
@@ -3103,7 +3173,7 @@ struct Fft
       float2 a[N1], b[N1];
 #pragma unroll
       for (int n1 = 0; n1 < N1; ++n1) a[n1] = in[N2 * n1 + n2];
-      Fft<N1>::run(a, b);
+      Fft<N1, kDirect>::run(a, b);
 #pragma unroll
       for (int k1 = 0; k1 < N1; ++k1) y[k1 * N2 + n2] = twiddle_mul<N>(b[k1], n2 * k1);
     }
@@ -3113,16 +3183,22 @@ struct Fft
       float2 a[N2], b[N2];
 #pragma unroll
       for (int n2 = 0; n2 < N2; ++n2) a[n2] = y[k1 * N2 + n2];
-      Fft<N2>::run(a, b);
+      Fft<N2, kDirect>::run(a, b);
 #pragma unroll
       for (int k2 = 0; k2 < N2; ++k2) out[k1 + N1 * k2] = b[k2];
     }
   }
 };
-template <int N>
-struct Fft<N, N>
+template <int N, bool kDirect>
+struct Fft<N, kDirect, N>
 {
-  __device__ __forceinline__ static void run(const float2 (&in)[N], float2 (&out)[N]) { Dft<N>::run(in, out); }
+  __device__ __forceinline__ static void run(const float2 (&in)[N], float2 (&out)[N]) 
+  {
+    if constexpr (N > 5 && !kDirect)
+      DftPaired<N>::run(in, out);
+    else
+      Dft<N>::run(in, out);
+  }
 };
 
 // Prime-factor (Good-Thomas) transform: N = N1 * N2 with gcd(N1, N2) = 1, N1 the full power
@@ -3149,7 +3225,7 @@ __host__ __device__ constexpr int inverse_mod(int a, int m)
   return 1;
 }
 
-template <int N, int N1 = prime_power_part(N)>
+template <int N, bool kDirect = false, int N1 = prime_power_part(N)>
 struct FftPfa
 {
   static constexpr int N2 = N / N1;
@@ -3164,7 +3240,7 @@ struct FftPfa
       float2 a[N1], b[N1];
 #pragma unroll
       for (int n1 = 0; n1 < N1; ++n1) a[n1] = in[(N2 * n1 + N1 * n2) % N];
-      Fft<N1>::run(a, b);
+      Fft<N1, kDirect>::run(a, b);
 #pragma unroll
       for (int k1 = 0; k1 < N1; ++k1) y[k1 * N2 + n2] = b[k1];
     }
@@ -3174,16 +3250,16 @@ struct FftPfa
       float2 a[N2], b[N2];
 #pragma unroll
       for (int n2 = 0; n2 < N2; ++n2) a[n2] = y[k1 * N2 + n2];
-      FftPfa<N2>::run(a, b);
+      FftPfa<N2, kDirect>::run(a, b);
 #pragma unroll
       for (int k2 = 0; k2 < N2; ++k2) out[(k1 * E1 + k2 * E2) % N] = b[k2];
     }
   }
 };
-template <int N>
-struct FftPfa<N, N>
+template <int N, bool kDirect>
+struct FftPfa<N, kDirect, N>
 {
-  __device__ __forceinline__ static void run(const float2 (&in)[N], float2 (&out)[N]) { Fft<N>::run(in, out); }
+  __device__ __forceinline__ static void run(const float2 (&in)[N], float2 (&out)[N]) { Fft<N, kDirect>::run(in, out); }
 };
 
 // --------------------------------------------------------------------------------------
@@ -3205,7 +3281,20 @@ struct FftccParams
   int w, h;
   const int64_t* n_dev = nullptr;   // device-side queue length (overrides n when set)
   const int* enable = nullptr;      // device-side switch: the launch does nothing when 0
+  // Near ties.  Two peaks of a map closer than the transforms' rounding fall either way with the
+  // order of its sums.  The kernels that use a cheaper order (k_fftcc_line, k_fftcc2 with a prime
+  // factor above 5) leave POIs with another value within kNearTie of their peak to a second launch
+  // over near[0 .. *near_n), which decides them in the plain order: the peak does not depend on
+  // which kernel is the faster one.
+  int64_t* near = nullptr;
+  unsigned long long* near_n = nullptr;
 };
+// Distance of two near-tied values over (rn + tn) / 2 M^2, the scale of the packed transform's
+// rounding (at rn = tn the value of a perfect match; a flat window's noise lies far below it).
+// The forms of a transform differ by at most 6.6e-7 of it, measured on 3.2 million POIs at radii
+// 7 to 32, u8 and offset float images.
+constexpr float kNearTie = 1e-5f;
+__device__ __forceinline__ void leave_near_tie(const FftccParams& P, int64_t i) { P.near[atomicAdd(P.near_n, 1ull)] = i; }
 
 template <int M>
 __global__ void __launch_bounds__(128) k_fftcc(FftccParams P)
@@ -3268,7 +3357,7 @@ __global__ void __launch_bounds__(128) k_fftcc(FftccParams P)
   {
 #pragma unroll
     for (int k = 0; k < M; ++k) a[k] = z[lane * S + k];
-    Fft<M>::run(a, b);
+    Fft<M, true>::run(a, b);
 #pragma unroll
     for (int k = 0; k < M; ++k) z[lane * S + k] = b[k];
   }
@@ -3278,7 +3367,7 @@ __global__ void __launch_bounds__(128) k_fftcc(FftccParams P)
   {
 #pragma unroll
     for (int k = 0; k < M; ++k) a[k] = z[k * S + lane];
-    Fft<M>::run(a, b);
+    Fft<M, true>::run(a, b);
   }
   __syncwarp();
   if (lane < M)
@@ -3303,7 +3392,7 @@ __global__ void __launch_bounds__(128) k_fftcc(FftccParams P)
       const float2 X = make_float2(Rk.x * Tk.x + Rk.y * Tk.y, Rk.x * Tk.y - Rk.y * Tk.x);
       a[k] = make_float2(X.x, -X.y);  // inverse via conj(FFT(conj(X)))
     }
-    Fft<M>::run(a, b);
+    Fft<M, true>::run(a, b);
   }
   __syncwarp();
   if (lane < M)
@@ -3318,7 +3407,7 @@ __global__ void __launch_bounds__(128) k_fftcc(FftccParams P)
   {
 #pragma unroll
     for (int k = 0; k < M; ++k) a[k] = z[lane * S + k];
-    Fft<M>::run(a, b);
+    Fft<M, true>::run(a, b);
     // real part of conj(FFT(conj(.))) is the real part of the FFT output
 #pragma unroll
     for (int k = 0; k < M; ++k)
@@ -3361,17 +3450,25 @@ __global__ void __launch_bounds__(128) k_fftcc(FftccParams P)
 #define DIC_FFTCC_INT_ROWS 1
 #endif
 constexpr bool kFftccIntRows = DIC_FFTCC_INT_ROWS != 0;
-template <int M>
-// (Register caps for 7 or 8 CTAs per SM spill: 0.93 against 0.67 ms at 2048^2.)
-__global__ void __launch_bounds__(64) k_fftcc2(FftccParams P)
+// A largest prime factor above 5 leaves near ties to the second pass (kSecond: over P.near, in the
+// plain order), see FftccParams::near.
+__host__ __device__ constexpr bool fftcc2_near(int m)
+{
+  for (int d = 7; d <= m; ++d)
+    if (m % d == 0 && is_prime(d)) return true;
+  return false;
+}
+// Two POIs on the calling warp: queue indices i0, i0 + 1, or (kSecond) the entries i0, i0 + 1 of
+// P.near, of which `listed` exist; zs: the warp's two windows.
+template <int M, bool kSecond>
+__device__ __forceinline__ void fftcc2_warp(const FftccParams& P, int64_t i0, int64_t listed, float2* zs)
 {
   static_assert(M % 2 == 0 && M / 2 + 1 <= 16, "16 inverse lanes per POI");
   constexpr int R = M / 2, S = M + 1;
-  constexpr int kWarps = 2;
-  __shared__ float2 smem[kWarps * 2][M * S];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t i0 = ((int64_t)blockIdx.x * kWarps + warp) * 2;
+  constexpr bool kNear = fftcc2_near(M) && !kSecond;
+  const int lane = threadIdx.x & 31;
   const int w = P.w, h = P.h;
+  const auto index = [&](int q) { return kSecond ? P.near[i0 + q] : i0 + q; };
   // per-POI scalars of the two POIs, kept as named registers (the POI loop is not unrolled,
   // which keeps one copy of the forward transforms in the instruction stream)
   bool live0 = false, live1 = false;
@@ -3382,8 +3479,9 @@ __global__ void __launch_bounds__(64) k_fftcc2(FftccParams P)
 #pragma unroll 1
   for (int q = 0; q < 2; ++q)
   {
-    const int64_t i = i0 + q;
-    bool lv = queue_slot_active(P, i);
+    const bool in = !kSecond || i0 + q < listed;
+    const int64_t i = in ? index(q) : 0;
+    bool lv = in && queue_slot_active(P, i);
     float ui = 0.f, vi = 0.f, px = 0.f, py = 0.f;
     if (lv)
     {
@@ -3399,7 +3497,7 @@ __global__ void __launch_bounds__(64) k_fftcc2(FftccParams P)
     if (q == 0) { live0 = lv; uq0 = ui; vq0 = vi; }
     else { live1 = lv; uq1 = ui; vq1 = vi; }
     if (!lv) continue;
-    float2* z = smem[warp * 2 + q];
+    float2* z = zs + q * (M * S);
     float rv[M], tv[M];
     float rsum = 0.f, tsum = 0.f;
     if (lane < M)
@@ -3448,7 +3546,7 @@ __global__ void __launch_bounds__(64) k_fftcc2(FftccParams P)
         tnl += tv[r] * tv[r];
         a[r] = make_float2(rv[r], tv[r]);
       }
-      FftPfa<M>::run(a, b);
+      FftPfa<M, kSecond>::run(a, b);
 #pragma unroll
       for (int k = 0; k < M; ++k) z[k * S + lane] = b[k];
     }
@@ -3460,7 +3558,7 @@ __global__ void __launch_bounds__(64) k_fftcc2(FftccParams P)
     {
 #pragma unroll
       for (int k = 0; k < M; ++k) a[k] = z[lane * S + k];
-      FftPfa<M>::run(a, b);
+      FftPfa<M, kSecond>::run(a, b);
 #pragma unroll
       for (int k = 0; k < M; ++k) z[lane * S + k] = b[k];
     }
@@ -3468,7 +3566,7 @@ __global__ void __launch_bounds__(64) k_fftcc2(FftccParams P)
   }
   // inverse columns c = 0..R of conj(X), X = conj(R) T, both POIs at once: lane -> (POI, c)
   const int q = lane >> 4, c = lane & 15;
-  float2* zq = smem[warp * 2 + q];
+  float2* zq = zs + q * (M * S);
   const bool live_q = q ? live1 : live0;
   const bool col_live = live_q && c <= R;
   if (col_live)
@@ -3486,7 +3584,7 @@ __global__ void __launch_bounds__(64) k_fftcc2(FftccParams P)
       const float2 X = make_float2(Rk.x * Tk.x + Rk.y * Tk.y, Rk.x * Tk.y - Rk.y * Tk.x);
       a[k] = make_float2(X.x, -X.y);
     }
-    FftPfa<M>::run(a, b);
+    FftPfa<M, kSecond>::run(a, b);
   }
   __syncwarp();   // every partner column is read before any column is overwritten
   if (col_live)
@@ -3521,7 +3619,7 @@ __global__ void __launch_bounds__(64) k_fftcc2(FftccParams P)
       }
       a[col] = make_float2(va.x - vb.y, va.y + vb.x);   // va + i vb
     }
-    FftPfa<M>::run(a, b);
+    FftPfa<M, kSecond>::run(a, b);
     // real part: row ra, imaginary part: row rb (ra first: lower row-major indices)
 #pragma unroll
     for (int k = 0; k < M; ++k)
@@ -3538,11 +3636,27 @@ __global__ void __launch_bounds__(64) k_fftcc2(FftccParams P)
     const int oi = __shfl_xor_sync(kFull, best_idx, o);
     if (ov > best || (ov == best && oi < best_idx)) { best = ov; best_idx = oi; }
   }
+  const float nq = q ? rn1 * tn1 : rn0 * tn0;
+  if constexpr (kNear)
+  {
+    // values within the margin of the peak: the peak alone, or the second pass decides
+    const float least = best - kNearTie * (0.5f * (q ? rn1 + tn1 : rn0 + tn0) * (float)(M * M));
+    int close = 0;
+    if (row_live)
+#pragma unroll
+      for (int k = 0; k < M; ++k) close += (b[k].x >= least) + (b[k].y >= least);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) close += __shfl_xor_sync(kFull, close, o);
+    if (close > 1 && P.near)
+    {
+      if (c == 0 && live_q) leave_near_tie(P, index(q));
+      return;
+    }
+  }
   if (c == 0 && live_q)
   {
     const float uq = q ? uq1 : uq0, vq = q ? vq1 : vq0;
-    const float nq = q ? rn1 * tn1 : rn0 * tn0;
-    dic_poi* poi = P.pois + i0 + q;
+    dic_poi* poi = P.pois + index(q);
     int lu = best_idx % M, lv = best_idx / M;
     if (lu > R) lu -= M;
     if (lv > R) lv -= M;
@@ -3552,6 +3666,27 @@ __global__ void __launch_bounds__(64) k_fftcc2(FftccParams P)
     poi->v0 = vq;
     poi->zncc = best / (sqrtf(nq) * (float)(M * M));
   }
+}
+
+template <int M, bool kSecond = false>
+// (Register caps for 7 or 8 CTAs per SM spill: 0.93 against 0.67 ms at 2048^2.)
+__global__ void __launch_bounds__(64) k_fftcc2(FftccParams P)
+{
+  constexpr int kWarps = 2, S = M + 1;
+  __shared__ float2 smem[kWarps * 2][M * S];
+  const int warp = threadIdx.x >> 5;
+  const int64_t first = ((int64_t)blockIdx.x * kWarps + warp) * 2;
+  if constexpr (kSecond)
+  {
+    const int64_t listed = (int64_t)*P.near_n;
+    for (int64_t k = first; k < listed; k += (int64_t)gridDim.x * kWarps * 2)
+    {
+      fftcc2_warp<M, true>(P, k, listed, smem[warp * 2]);
+      __syncwarp();
+    }
+  }
+  else
+    fftcc2_warp<M, false>(P, first, 0, smem[warp * 2]);
 }
 
 // --------------------------------------------------------------------------------------
@@ -3649,7 +3784,7 @@ __device__ void dft_lines(const float2* in, float2* out, int m, int s, bool by_r
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(256) k_fftcc_large(FftccParams P, int m)
+__device__ __forceinline__ void fftcc_large_poi(const FftccParams& P, int m, int64_t i)
 {
   extern __shared__ float2 dyn[];
   __shared__ float s_red[32];
@@ -3657,8 +3792,6 @@ __global__ void __launch_bounds__(256) k_fftcc_large(FftccParams P, int m)
   const int s = m + 1;
   float2* za = dyn;
   float2* zb = dyn + m * s;
-  const int64_t i = blockIdx.x;
-  if (!queue_slot_active(P, i)) return;
   dic_poi* poi = P.pois + i;
   const float px = poi->x, py = poi->y, u_init = poi->u, v_init = poi->v;
   const int w = P.w, h = P.h, R = m / 2;
@@ -3732,6 +3865,22 @@ __global__ void __launch_bounds__(256) k_fftcc_large(FftccParams P, int m)
   }
 }
 
+// one CTA per POI of the queue, or (near) the POIs of P.near
+__global__ void __launch_bounds__(256) k_fftcc_large(FftccParams P, int m)
+{
+  if (!P.near)
+  {
+    if (queue_slot_active(P, (int64_t)blockIdx.x)) fftcc_large_poi(P, m, blockIdx.x);
+    return;
+  }
+  const int64_t listed = (int64_t)*P.near_n;
+  for (int64_t k = blockIdx.x; k < listed; k += gridDim.x)
+  {
+    fftcc_large_poi(P, m, P.near[k]);
+    __syncthreads();
+  }
+}
+
 // --------------------------------------------------------------------------------------
 // FFTCC for 32 < M <= 64 (subset radius 17..32) as a real FFT: one 128-thread CTA per POI,
 // the packed window z = ref + i tar in shared memory ([M][M + 1] float2; consecutive lanes
@@ -3777,7 +3926,7 @@ __device__ __forceinline__ void big_forward(float2* z, int line, int part, bool 
       float2 a[N1], b[N1];
 #pragma unroll
       for (int n1 = 0; n1 < N1; ++n1) a[n1] = z[line_at<M, kRows>(line, N2 * n1 + n2)];
-      Fft<N1>::run(a, b);
+      Fft<N1, true>::run(a, b);
 #pragma unroll
       for (int k1 = 0; k1 < N1; ++k1) z[line_at<M, kRows>(line, N2 * k1 + n2)] = k1 ? cmul(b[k1], tw[n2 * k1]) : b[k1];
     }
@@ -3788,7 +3937,7 @@ __device__ __forceinline__ void big_forward(float2* z, int line, int part, bool 
       float2 a[N2], b[N2];
 #pragma unroll
       for (int n2 = 0; n2 < N2; ++n2) a[n2] = z[line_at<M, kRows>(line, N2 * k1 + n2)];
-      Fft<N2>::run(a, b);
+      Fft<N2, true>::run(a, b);
 #pragma unroll
       for (int k2 = 0; k2 < N2; ++k2) z[line_at<M, kRows>(line, N2 * k1 + k2)] = b[k2];
     }
@@ -3807,7 +3956,7 @@ __device__ __forceinline__ void big_from_permuted(float2* z, int line, int part,
       float2 a[N2], b[N2];
 #pragma unroll
       for (int k2 = 0; k2 < N2; ++k2) a[k2] = z[line_at<M, kRows>(line, N2 * k1 + k2)];
-      Fft<N2>::run(a, b);
+      Fft<N2, true>::run(a, b);
 #pragma unroll
       for (int j = 0; j < N2; ++j) z[line_at<M, kRows>(line, N2 * k1 + j)] = k1 ? cmul(b[j], tw[j * k1]) : b[j];
     }
@@ -3818,7 +3967,7 @@ __device__ __forceinline__ void big_from_permuted(float2* z, int line, int part,
       float2 a[N1], b[N1];
 #pragma unroll
       for (int k1 = 0; k1 < N1; ++k1) a[k1] = z[line_at<M, kRows>(line, N2 * k1 + j)];
-      Fft<N1>::run(a, b);
+      Fft<N1, true>::run(a, b);
 #pragma unroll
       for (int i = 0; i < N1; ++i) z[line_at<M, kRows>(line, N2 * i + j)] = b[i];
     }
@@ -3826,15 +3975,13 @@ __device__ __forceinline__ void big_from_permuted(float2* z, int line, int part,
 }
 
 template <int M>
-__global__ void __launch_bounds__(kBigThreads) k_fftcc_big(FftccParams P)
+__device__ __forceinline__ void fftcc_big_poi(const FftccParams& P, int64_t i)
 {
   constexpr int N1 = big_n1(M), N2 = M / N1, S = M + 1, R = M / 2, kParts = kBigThreads / M;
   static_assert(kParts >= 1, "one thread per line at least");
   extern __shared__ float2 zbig[];
   __shared__ float s_red[32];
   __shared__ int s_idx[32];
-  const int64_t i = blockIdx.x;
-  if (!queue_slot_active(P, i)) return;
   dic_poi* poi = P.pois + i;
   const float px = poi->x, py = poi->y, u_init = poi->u, v_init = poi->v;
   const int w = P.w, h = P.h;
@@ -3924,6 +4071,394 @@ __global__ void __launch_bounds__(kBigThreads) k_fftcc_big(FftccParams P)
     poi->u0 = u_init;
     poi->v0 = v_init;
     poi->zncc = best / (sqrtf(rn * tn) * (float)(M * M));
+  }
+}
+
+// the POIs of P.near, in the plain order
+template <int M>
+__global__ void __launch_bounds__(kBigThreads) k_fftcc_big(FftccParams P)
+{
+  const int64_t listed = (int64_t)*P.near_n;
+  for (int64_t k = blockIdx.x; k < listed; k += gridDim.x)
+  {
+    fftcc_big_poi<M>(P, P.near[k]);
+    __syncthreads();
+  }
+}
+
+// --------------------------------------------------------------------------------------
+// FFTCC for 32 < M <= 64 (subset radius 17..32): the packed window z = ref + i tar of a POI in
+// shared memory ([M][M + 1] float2; consecutive lanes take consecutive lines, whose odd float2
+// stride keeps a warp's accesses conflict-free in both directions), one thread per line, kPois
+// POIs per CTA so that the lines fill its warps.  A thread transforms its line in place in two
+// stages of small register FFTs, all positions compile-time constants:
+//   M = N1 x N2 coprime (every M here but 64): the prime-factor form.  Slot (i1, i2) of a line
+//   is position (N2 i1 + N1 i2) mod M; a transform over i1 and one over i2, no twiddles between,
+//   takes a line in natural order to one whose slot (k1, k2) holds the bin k = k1 (mod N1), k2
+//   (mod N2) -- and such a line back to natural order.
+//   M = 64: four-step 8 x 8 with twiddles, slot (i1, i2) = 8 i1 + i2, bin k1 + 8 k2.
+// Columns (zero-mean values formed on the way), rows; then the cross-power conj(R) T and the way
+// back on half the lines: the correlation is real, so only the columns 0..M/2 of conj(X) are
+// transformed, and the rows j and j + M/2 go through one complex row transform as its real and
+// imaginary parts (as in k_fftcc2).  Argmax with the CPU's tie rule: the POI's maximum first, its
+// lowest index from the rows that hold it.
+//
+// Bound by instruction issue.  k_fftcc_big (128 threads a POI, lines split over threads, a runtime
+// index and a table twiddle per element, all lines on the way back) issues 2.5 times the
+// instructions; lengths 2 x prime ran as direct DFTs (k_fftcc_large).  Both remain for near ties.
+// Before and now: r 20, 29 000 POIs 0.315 -> 0.208 ms; r 30, 36 864 POIs 0.89 -> 0.70 ms; r 31,
+// 9 396 POIs 1.85 -> 0.39 ms; r 17, 30 000 POIs 2.18 -> 0.25 ms.  (k_fftcc2<14> with the paired
+// 7-point DFT, 171 024 POIs: 0.32 -> 0.20 ms.)
+// --------------------------------------------------------------------------------------
+__host__ __device__ constexpr int gcd(int a, int b) { return b ? gcd(b, a % b) : a; }
+__host__ __device__ constexpr int line_n1(int m)
+{
+  int best = 0;   // the smaller factor of the most even coprime split, else 8 (64)
+  for (int d = 2; d * d <= m; ++d)
+    if (m % d == 0 && gcd(d, m / d) == 1) best = d;
+  return best ? best : 8;
+}
+template <int M>
+struct LinePlan
+{
+  static constexpr int N1 = line_n1(M), N2 = M / N1, S = M + 1, R = M / 2;
+  static constexpr bool kPfa = gcd(N1, N2) == 1;
+  static_assert(N1 * N2 == M, "line split");
+  static constexpr int E1 = N2 * inverse_mod(N2 % N1, N1), E2 = N1 * inverse_mod(N1 % N2, N2);
+  __host__ __device__ static constexpr int slot(int i1, int i2) { return kPfa ? (N2 * i1 + N1 * i2) % M : N2 * i1 + i2; }
+  // M = 2 N2 with a prime N2 >= 17: the two length-N2 transforms of a line share one copy of
+  // their code (some 900 FMAs at 31; four such lines' copies overflow the instruction cache).
+  // slot (loop + g, i2) with a runtime loop: slot(1, i2) lies N2 after or before slot(0, i2)
+  static constexpr bool kLoop = N1 == 2 && N2 >= 17 && is_prime(N2);
+  __device__ __forceinline__ static int slot_at(int loop, int g, int i2)
+  {
+    if constexpr (kLoop)
+    {
+      const int d = loop ? N2 : 0;
+      return slot(0, i2) + (slot(1, i2) > slot(0, i2) ? d : -d);
+    }
+    else
+      return slot(g, i2);
+  }
+  __host__ __device__ static constexpr int bin(int k1, int k2) { return kPfa ? (k1 * E1 + k2 * E2) % M : k1 + N1 * k2; }
+  __host__ __device__ static constexpr int pos(int k) { return kPfa ? slot(k % N1, k % N2) : slot(k % N1, k / N1); }
+};
+
+// forward transform of a line in place; ld(position) reads an element, element e at z[e * kStep]
+template <int M, int kStep, class Ld>
+__device__ __forceinline__ void line_forward(float2* z, Ld ld)
+{
+  using L = LinePlan<M>;
+  constexpr int N1 = L::N1, N2 = L::N2;
+#pragma unroll
+  for (int i2 = 0; i2 < N2; ++i2)
+  {
+    float2 a[N1], b[N1];
+#pragma unroll
+    for (int i1 = 0; i1 < N1; ++i1) a[i1] = ld(L::slot(i1, i2));
+    FftPfa<N1>::run(a, b);
+#pragma unroll
+    for (int k1 = 0; k1 < N1; ++k1)
+      z[L::slot(k1, i2) * kStep] = L::kPfa ? b[k1] : twiddle_mul<M>(b[k1], i2 * k1);
+  }
+  constexpr int kGroups = L::kLoop ? 1 : N1;   // unrolled copies of the second stage
+#pragma unroll 1
+  for (int loop = 0; loop < N1; loop += kGroups)
+#pragma unroll
+    for (int g = 0; g < kGroups; ++g)
+    {
+      float2 a[N2], b[N2];
+#pragma unroll
+      for (int i2 = 0; i2 < N2; ++i2) a[i2] = z[L::slot_at(loop, g, i2) * kStep];
+      FftPfa<N2>::run(a, b);
+#pragma unroll
+      for (int k2 = 0; k2 < N2; ++k2) z[L::slot_at(loop, g, k2) * kStep] = b[k2];
+    }
+}
+// the same transform of a line of bins, back to natural order: ld.bin(k) gives bin k, ld.at(k1, k2)
+// with a runtime k1 the bin of slot (k1, k2).  Bins k and -k are read together before either's
+// slots are written (k1 with its mirror N1 - k1).
+// st(n, value) takes the results.
+template <int M, int kStep, class Ld, class St>
+__device__ __forceinline__ void line_back(float2* z, Ld ld, St st)
+{
+  using L = LinePlan<M>;
+  constexpr int N1 = L::N1, N2 = L::N2;
+  if constexpr (L::kLoop)
+  {
+    // k1 = 0 and 1 are their own mirrors
+#pragma unroll 1
+    for (int loop = 0; loop < 2; ++loop)
+    {
+      float2 a[N2], b[N2];
+#pragma unroll
+      for (int k2 = 0; k2 < N2; ++k2) a[k2] = ld.at(loop, k2);
+      FftPfa<N2>::run(a, b);
+#pragma unroll
+      for (int j = 0; j < N2; ++j) z[L::slot_at(loop, 0, j) * kStep] = b[j];
+    }
+  }
+  else
+  {
+#pragma unroll
+    for (int k1 = 0; k1 <= N1 / 2; ++k1)
+    {
+      const int m1 = (N1 - k1) % N1;
+      float2 a[N2], c[N2], b[N2];
+#pragma unroll
+      for (int k2 = 0; k2 < N2; ++k2)
+      {
+        a[k2] = ld.bin(L::bin(k1, k2));
+        if (m1 != k1) c[k2] = ld.bin(L::bin(m1, k2));
+      }
+      FftPfa<N2>::run(a, b);
+#pragma unroll
+      for (int j = 0; j < N2; ++j) z[L::slot(k1, j) * kStep] = L::kPfa ? b[j] : twiddle_mul<M>(b[j], j * k1);
+      if (m1 != k1)
+      {
+        FftPfa<N2>::run(c, b);
+#pragma unroll
+        for (int j = 0; j < N2; ++j) z[L::slot(m1, j) * kStep] = L::kPfa ? b[j] : twiddle_mul<M>(b[j], j * m1);
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < N2; ++j)
+  {
+    float2 a[N1], b[N1];
+#pragma unroll
+    for (int k1 = 0; k1 < N1; ++k1) a[k1] = z[L::slot(k1, j) * kStep];
+    FftPfa<N1>::run(a, b);
+#pragma unroll
+    for (int i = 0; i < N1; ++i) st(L::slot(i, j), b[i]);
+  }
+}
+
+// bins of a column of conj(X), X = conj(R) T, from Z's column (zj) and its mirror column (zm)
+template <int M>
+struct CrossPower
+{
+  using L = LinePlan<M>;
+  const float2 *zj, *zm;
+  __device__ __forceinline__ static float2 of(float2 A, float2 m)
+  {
+    const float2 B = make_float2(m.x, -m.y);
+    const float2 Rk = make_float2(0.5f * (A.x + B.x), 0.5f * (A.y + B.y));
+    const float2 D = csub(A, B);
+    const float2 Tk = make_float2(0.5f * D.y, -0.5f * D.x);   // D / (2i)
+    return make_float2(Rk.x * Tk.x + Rk.y * Tk.y, Rk.y * Tk.x - Rk.x * Tk.y);
+  }
+  __device__ __forceinline__ float2 bin(int k) const { return of(zj[L::pos(k) * L::S], zm[L::pos((M - k) % M) * L::S]); }
+  __device__ __forceinline__ float2 at(int k1, int k2) const
+  {
+    return of(zj[L::slot_at(k1, 0, k2) * L::S], zm[L::slot_at(k1, 0, (L::N2 - k2) % L::N2) * L::S]);
+  }
+};
+// bins of rows a + i b, the columns past M/2 as the conjugate mirrors of the others
+template <int M>
+struct RowPair
+{
+  using L = LinePlan<M>;
+  const float2 *za, *zb;
+  __device__ __forceinline__ static float2 of(float2 va, float2 vb, bool mirror)
+  {
+    if (mirror)
+    {
+      va.y = -va.y;
+      vb.y = -vb.y;
+    }
+    return make_float2(va.x - vb.y, va.y + vb.x);
+  }
+  __device__ __forceinline__ float2 bin(int k) const
+  {
+    const int c = k <= L::R ? k : M - k;
+    return of(za[L::pos(c)], zb[L::pos(c)], k > L::R);
+  }
+  __device__ __forceinline__ float2 at(int k1, int k2) const
+  {
+    const int k = k1 ? L::bin(1, k2) : L::bin(0, k2), p = k <= L::R ? L::slot_at(k1, 0, k2)
+                                                                  : L::slot_at(k1, 0, (L::N2 - k2) % L::N2);
+    return of(za[p], zb[p], k > L::R);
+  }
+};
+
+template <int M, int kPois>
+struct FftccLine
+{
+  static constexpr int kThreads = (kPois * M + 31) / 32 * 32;
+  static constexpr size_t kSmem = (size_t)kPois * M * (M + 1) * sizeof(float2);
+};
+template <int M, int kPois>
+__global__ void __launch_bounds__(FftccLine<M, kPois>::kThreads) k_fftcc_line(FftccParams P)
+{
+  using L = LinePlan<M>;
+  constexpr int S = L::S, R = L::R, kThreads = FftccLine<M, kPois>::kThreads;
+  extern __shared__ __align__(16) float2 zline[];
+  __shared__ float2 s_part[kThreads], s_eight[kPois * 8];
+  __shared__ float s_max[kPois][R], s_top[kPois], s_margin[kPois];
+  __shared__ int s_idx[kPois], s_live[kPois], s_close[kPois];
+  const int tid = threadIdx.x;
+  const int w = P.w, h = P.h;
+  const int q = tid / M, c = tid % M;
+  const int64_t i = (int64_t)blockIdx.x * kPois + q;
+  if (!queue_slot_active(P, (int64_t)blockIdx.x * kPois)) return;   // the whole CTA
+  // a POI's threads decide alike; out-of-range POIs are left untouched, as the CPU leaves them
+  float px = 0.f, py = 0.f, ui = 0.f, vi = 0.f;
+  bool on = q < kPois && queue_slot_active(P, i);
+  if (on)
+  {
+    const dic_poi* poi = P.pois + i;
+    px = poi->x;
+    py = poi->y;
+    ui = poi->u;
+    vi = poi->v;
+    on = !((int)px < R || (int)px >= w - R || (int)py < R || (int)py >= h - R || int(px + ui) < R ||
+           int(px + ui) >= w - R || int(py + vi) < R || int(py + vi) >= h - R);
+  }
+  if (q < kPois && c == 0) s_live[q] = on;
+  float2* z = zline + q * (M * S);
+  float2 sum = make_float2(0.f, 0.f);
+  if (on)
+  {
+    const float fxr = __fsub_rn(__fadd_rn(px, (float)c), (float)R);
+    const int xr = (int)fxr, xt = (int)__fadd_rn(fxr, ui);
+    if (py == rintf(py) && vi == rintf(vi))
+    {
+      // whole-pixel row coordinate and seed: the CPU's float row coordinates are exact
+      const float* rp = P.ref + (size_t)((int)py - R) * w + xr;
+      const float* tp = P.tar + (size_t)((int)py - R + (int)vi) * w + xt;
+#pragma unroll 8
+      for (int r = 0; r < M; ++r)
+      {
+        const float2 v = make_float2(__ldg(rp), __ldg(tp));
+        rp += w;
+        tp += w;
+        z[r * S + c] = v;
+        sum = cadd(sum, v);
+      }
+    }
+    else
+#pragma unroll 4
+      for (int r = 0; r < M; ++r)
+      {
+        const float fyr = __fsub_rn(__fadd_rn(py, (float)r), (float)R);
+        const float2 v = make_float2(P.ref[(size_t)(int)fyr * w + xr], P.tar[(size_t)(int)__fadd_rn(fyr, vi) * w + xt]);
+        z[r * S + c] = v;
+        sum = cadd(sum, v);
+      }
+  }
+  // sums over a POI's columns: eight threads add every eighth, every thread adds the eight
+  const auto poi_sum = [&](float2 v) {
+    s_part[tid] = v;
+    __syncthreads();
+    if (tid < kPois * 8)
+    {
+      float2 t = make_float2(0.f, 0.f);
+      for (int k = tid & 7; k < M; k += 8) t = cadd(t, s_part[(tid >> 3) * M + k]);
+      s_eight[tid] = t;
+    }
+    __syncthreads();
+    float2 t = make_float2(0.f, 0.f);
+    if (q < kPois)
+#pragma unroll
+      for (int k = 0; k < 8; ++k) t = cadd(t, s_eight[q * 8 + k]);
+    return t;
+  };
+  const float2 total = poi_sum(sum);
+  const float2 mean = make_float2(total.x / (float)(M * M), total.y / (float)(M * M));
+  float2 norm = make_float2(0.f, 0.f);
+  if (on)
+    line_forward<M, S>(z + c, [&](int r) {
+      const float2 v = csub(z[r * S + c], mean);
+      norm = __ffma2_rn(v, v, norm);
+      return v;
+    });
+  norm = poi_sum(norm);   // its barriers also end the column pass
+  if (on) line_forward<M, 1>(z + c * S, [&](int k) { return z[c * S + k]; });
+  if (tid < kPois)
+  {
+    s_idx[tid] = INT_MAX;
+    s_close[tid] = 0;
+  }
+  if (on && c == 0) s_margin[q] = kNearTie * (0.5f * (norm.x + norm.y) * (float)(M * M));
+  __syncthreads();
+  // From here a line's thread has another place: columns 0..R, then rows 0..R-1 of POI qb.
+  {
+    const int qb = tid / (R + 1), j = tid % (R + 1);
+    if (qb < kPois && s_live[qb])
+    {
+      // column kc = j of conj(X), X = conj(R) T from Z(k) and Z(-k); only this thread reads the
+      // mirror column's bins, and columns past R are not written
+      float2* zb = zline + qb * (M * S);
+      int pj = 0, pm = 0;   // positions of bins j and -j in a row
+      if constexpr (L::kPfa)
+      {
+        pj = (L::N2 * (j % L::N1) + L::N1 * (j % L::N2)) % M;
+        pm = (M - pj) % M;
+      }
+      else
+      {
+        const int mj = (M - j) % M;
+        pj = L::N2 * (j % L::N1) + j / L::N1;
+        pm = L::N2 * (mj % L::N1) + mj / L::N1;
+      }
+      line_back<M, S>(zb + pj, CrossPower<M>{zb + pj, zb + pm},
+                      [&](int n, float2 v) { zb[pj + n * S] = v; });
+    }
+  }
+  __syncthreads();
+  const int qb = tid / R, j = tid % R;
+  const bool row_on = qb < kPois && s_live[qb];
+  float2* za = zline + qb * (M * S) + j * S;   // rows j and j + R
+  float best = -2.f;
+  if (row_on)
+  {
+    line_back<M, 1>(
+        za, RowPair<M>{za, za + R * S},
+        [&](int n, float2 v) {
+          za[n] = v;
+          best = fmaxf(best, fmaxf(v.x, v.y));
+        });
+    s_max[qb][j] = best;
+  }
+  __syncthreads();
+  if (row_on)
+  {
+    float top = -2.f;
+#pragma unroll 6
+    for (int k = 0; k < R; ++k) top = fmaxf(top, s_max[qb][k]);
+    const float least = top - s_margin[qb];
+    if (best >= least)
+    {
+      int idx = INT_MAX, close = 0;
+      for (int n = 0; n < M; ++n)
+      {
+        const float2 v = za[n];
+        close += (v.x >= least) + (v.y >= least);
+        if (v.x == top) idx = min(idx, j * M + n);
+        if (v.y == top) idx = min(idx, (j + R) * M + n);
+      }
+      atomicMin(&s_idx[qb], idx);
+      atomicAdd(&s_close[qb], close);
+    }
+    if (j == 0) s_top[qb] = top;
+  }
+  __syncthreads();
+  if (on && c == 0 && s_close[q] > 1 && P.near)
+    leave_near_tie(P, i);
+  else if (on && c == 0)
+  {
+    dic_poi* poi = P.pois + i;
+    const float top = s_top[q];
+    const int idx = s_idx[q] == INT_MAX ? 0 : s_idx[q];
+    int lu = idx % M, lv = idx / M;
+    if (lu > R) lu -= M;
+    if (lv > R) lv -= M;
+    poi->u = (float)lu + ui;
+    poi->v = (float)lv + vi;
+    poi->u0 = ui;
+    poi->v0 = vi;
+    poi->zncc = top / (sqrtf(norm.x * norm.y) * (float)(M * M));
   }
 }
 
