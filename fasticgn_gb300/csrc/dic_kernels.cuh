@@ -1225,17 +1225,21 @@ __device__ __forceinline__ unsigned px_base()
 // the window (window_covers): the lane's nine sums, rows in order.  A row's 4 x 4 support
 // overlaps the one of the row before it in three rows of pixels, as long as both start in the
 // same column one row apart: those twelve pixels stay in registers (q, whose rows rotate by
-// unrolling) and a row loads four.  Where a lane's support steps otherwise (its warped column
-// or row crosses a pixel boundary) the warp reloads the other twelve (a third of the rows at
-// 1 % strain).  The rows go in groups of four without tests inside; a subset has an odd number
-// of rows, so the last group has three or one.  `mask`: the calling lanes.
+// unrolling) and a row loads four.  The rows go in groups of four: the addresses of a group's
+// samples come first, and where a lane's support steps otherwise in one of them (its warped
+// column or row crosses a pixel boundary) the warp loads all sixteen pixels of the group's
+// samples (kPerRow: the other twelve of the rows where one does; with two POIs in a warp whole
+// groups without a crossing are rarer).  A subset has an odd number of rows, so the last group has three or one.  `mask`: the
+// calling lanes.
 //
-// What bounds it: issue slots (98 instructions a row before, 86 now, of which 24 are the weights'
-// twelve packed products, two slots of the FMA pipe each) and the reference texel's trip to L2.
-// 96 registers hold a whole group in flight, so 20 resident warps do better than the 32 that
-// 64 registers allowed (2.86 against 3.18 ms of IC-GN on a 2048x2048 pair, 254 016 POIs, with
-// the lattice loop below; 24 warps 2.85, 16 warps 3.1).  Prefetching the texel a row ahead,
-// scalar weights and a packed form of add_sample moved the time by 1 % or less either way.
+// What bounds it: issue slots (98 instructions a row when every row loaded sixteen pixels, of
+// which 24 are the weights' twelve packed products, two slots of the FMA pipe each) and the
+// reference texels' trip to L2, so a group's four texels are loaded before anything else.  96
+// registers hold a group in flight: 20 resident warps do better than the 32 that 64 registers
+// allowed.  IC-GN on a 2048x2048 pair, 254 016 POIs, r 15: 3.18 -> 2.75 ms with the lattice loop
+// below (with a test per row instead of one per group 2.86, with the texels loaded first 2.79;
+// 16 warps 2.90, 24 warps 2.87); r 30, 36 864 POIs 1.31 -> 1.00 (28 warps 1.11); r 7, two POIs a
+// warp, 171 024 POIs: 0.71 with a test per row, 0.73 per group.  Scalar weights and packed sums moved the time by 1 % or less either way.
 struct ColumnRows
 {
   float q[4][4];
@@ -1245,45 +1249,82 @@ struct ColumnRows
   float t0;
   int w;
 };
-template <int kN>
+template <int kN, bool kPerRow>
 __device__ __forceinline__ void px_row_group(ColumnRows& S, ColumnSums& c)
 {
+  float4 texel[kN];
 #pragma unroll
   for (int k = 0; k < kN; ++k)
   {
-    const float4 cur = __ldg(S.rp);
+    texel[k] = __ldg(S.rp);
     S.rp += S.w;
-    const float2 g = __fadd2_rn(S.pxy, __ffma2_rn(S.Wy, S.fly, S.axy));
-    const float2 bits = floor_bits2(g);
-    const float2 d = csub(g, __fadd2_rn(bits, k2(-kFloorMagic)));
-    const unsigned a = S.org + 4u * __float_as_uint(bits.x) + S.pitch * __float_as_uint(bits.y);
-    const unsigned last = a + 3 * S.pitch;
-    if (!__all_sync(S.mask, a == S.expect))
-    {
-      // keeps this a branch: as predicated loads the twelve cost their issue slots every row
-      asm volatile("bar.warp.sync %0;" ::"r"(S.mask));
+  }
+  float2 d[kN];
+  unsigned a[kN];
+  bool steady[kN], all_steady = true;
+  float2 fly = S.fly;
 #pragma unroll
-      for (int n = 0; n < 3; ++n)
-      {
-        const unsigned b = a + n * S.pitch;
-        S.q[(n + k) & 3][0] = px_at<0>(b);
-        S.q[(n + k) & 3][1] = px_at<4>(b);
-        S.q[(n + k) & 3][2] = px_at<8>(b);
-        S.q[(n + k) & 3][3] = px_at<12>(b);
-      }
-    }
-    S.q[(3 + k) & 3][0] = px_at<0>(last);
-    S.q[(3 + k) & 3][1] = px_at<4>(last);
-    S.q[(3 + k) & 3][2] = px_at<8>(last);
-    S.q[(3 + k) & 3][3] = px_at<12>(last);
-    S.expect = a + S.pitch;
+  for (int k = 0; k < kN; ++k)
+  {
+    const float2 g = __fadd2_rn(S.pxy, __ffma2_rn(S.Wy, fly, S.axy));
+    const float2 bits = floor_bits2(g);
+    d[k] = csub(g, __fadd2_rn(bits, k2(-kFloorMagic)));
+    a[k] = S.org + 4u * __float_as_uint(bits.x) + S.pitch * __float_as_uint(bits.y);
+    steady[k] = a[k] == S.expect;
+    all_steady = all_steady && steady[k];
+    S.expect = a[k] + S.pitch;
+    fly = __fadd2_rn(fly, k2(1.f));
+  }
+  const auto load_row = [&](int at, unsigned b) {
+    S.q[at & 3][0] = px_at<0>(b);
+    S.q[at & 3][1] = px_at<4>(b);
+    S.q[at & 3][2] = px_at<8>(b);
+    S.q[at & 3][3] = px_at<12>(b);
+  };
+  const auto sample = [&](int k) {
     float2 wt[4];
-    bspline_weights2(d, wt);
+    bspline_weights2(d[k], wt);
     const float t = eval_pixels(wt, [&](int n, int m) { return S.q[(n + k) & 3][m]; });
-    add_sample(c, t, cur, S.t0, S.fly.x);
+    add_sample(c, t, texel[k], S.t0, S.fly.x);
     S.fly = __fadd2_rn(S.fly, k2(1.f));
+  };
+  if constexpr (kPerRow)
+  {
+#pragma unroll
+    for (int k = 0; k < kN; ++k)
+    {
+      if (!__all_sync(S.mask, steady[k]))
+      {
+        // keeps this a branch: as predicated loads the twelve cost their issue slots every row
+        asm volatile("bar.warp.sync %0;" ::"r"(S.mask));
+#pragma unroll
+        for (int n = 0; n < 3; ++n) load_row(n + k, a[k] + n * S.pitch);
+      }
+      load_row(3 + k, a[k] + 3 * S.pitch);
+      sample(k);
+    }
+  }
+  else if (__all_sync(S.mask, all_steady))
+  {
+#pragma unroll
+    for (int k = 0; k < kN; ++k)
+    {
+      load_row(3 + k, a[k] + 3 * S.pitch);
+      sample(k);
+    }
+  }
+  else
+  {
+#pragma unroll
+    for (int k = 0; k < kN; ++k)
+    {
+#pragma unroll
+      for (int n = 0; n < 4; ++n) load_row(n + k, a[k] + n * S.pitch);
+      sample(k);
+    }
   }
 }
+template <bool kPerRow>
 __device__ __forceinline__ void px_column_rows(ColumnSums& c, const PixelTile& T, const float4* __restrict__ rp, int w,
                                                float2 pxy, float2 axy, float2 Wy, float t0, int ry, unsigned mask)
 {
@@ -1302,11 +1343,11 @@ __device__ __forceinline__ void px_column_rows(ColumnSums& c, const PixelTile& T
   S.w = w;
   S.rp = rp;
 #pragma unroll 1
-  for (int r = (2 * ry + 1) >> 2; r > 0; --r) px_row_group<4>(S, c);
+  for (int r = (2 * ry + 1) >> 2; r > 0; --r) px_row_group<4, kPerRow>(S, c);
   if (ry & 1)
-    px_row_group<3>(S, c);
+    px_row_group<3, kPerRow>(S, c);
   else
-    px_row_group<1>(S, c);
+    px_row_group<1, kPerRow>(S, c);
 }
 
 // The same for an iteration on the pixel lattice (on_lattice: the first one from an FFTCC
@@ -1332,6 +1373,7 @@ __device__ __noinline__ ColumnSums px_column_lattice(int src, int pitch, const f
 
 // One column's sums of an iteration: lane column flx under warp W, in the form the iteration
 // allows (covered: window_covers, lat: on_lattice, both warp-uniform).
+template <bool kPerRow = false>
 __device__ __forceinline__ ColumnSums px_column(const PixelTile& T, const float* __restrict__ tar,
                                                 const float4* __restrict__ ref_col, int w, int h, float px, float py,
                                                 const float (&W)[6], float flx, float t0, int ry, bool covered, bool lat,
@@ -1345,7 +1387,7 @@ __device__ __forceinline__ ColumnSums px_column(const PixelTile& T, const float*
     c = px_column_lattice(T.s + ((int)(py + fmaf(W[4], (float)-ry, ay)) - T.oy) * T.bx + ((int)(px + ax) - T.ox), T.bx,
                           ref_col, w, t0, ry);
   else
-    px_column_rows(c, T, ref_col, w, make_float2(px, py), make_float2(ax, ay), make_float2(W[1], W[4]), t0, ry, mask);
+    px_column_rows<kPerRow>(c, T, ref_col, w, make_float2(px, py), make_float2(ax, ay), make_float2(W[1], W[4]), t0, ry, mask);
   return c;
 }
 
@@ -1579,10 +1621,8 @@ constexpr int icgn_min_blocks(int warps) { return DIC_ICGN_RESIDENT_WARPS / warp
 #define DIC_ICGN_PERSISTENT_RESIDENT_WARPS 32
 #endif
 constexpr int icgn_persistent_min_blocks(int warps) { return DIC_ICGN_PERSISTENT_RESIDENT_WARPS / warps; }
-// The pixel-window kernels: 20 resident warps (96 registers) for the column walk, 28 (72) for
-// the pair walk, whose windows leave room for no more above r 20.
+// The pixel-window kernels' resident warps (px_column_rows): 20, 96 registers.
 constexpr int px_min_blocks(int warps) { return 20 / warps; }
-constexpr int pair_px_min_blocks(int warps) { return 28 / warps; }
 
 template <bool kColumn, int kWarps = 4>
 __global__ void __launch_bounds__(kWarps * 32, icgn_min_blocks(kWarps)) k_icgn(IcgnParams P)
@@ -2539,7 +2579,7 @@ __device__ __forceinline__ void icgn_solve_px_half(const IcgnParams& P, int64_t 
     const bool covered = window_covers(W, px, py, rx, ry, xmax, ymax, T, h16, half);
     const bool lat = on_lattice(W, px, py), col = run && h16 < sw;
     const unsigned rows = __ballot_sync(kFull, col && covered && !lat);
-    if (col) c = px_column(T, P.tar, ref_col, w, h, px, py, W, flx, t0, ry, covered, lat, rows);
+    if (col) c = px_column<true>(T, P.tar, ref_col, w, h, px, py, W, flx, t0, ry, covered, lat, rows);
     __syncwarp();
     const unsigned bad = __ballot_sync(kFull, c.bad != 0);
     if (bad)
@@ -2717,7 +2757,7 @@ __device__ __forceinline__ int64_t pair_fetch(unsigned long long* next, long lon
 // kMode as in k_icgn_px (2 TMA, 1 warp copies, 0 no windows).  Same bits for every kPoiWarps,
 // kWarps and kMode.
 template <int kPoiWarps, int kWarps, int kMode>
-__global__ void __launch_bounds__(kWarps * 32, pair_px_min_blocks(kWarps))
+__global__ void __launch_bounds__(kWarps * 32, px_min_blocks(kWarps))
     k_icgn_pair_px(IcgnParams P, const __grid_constant__ CUtensorMap map, unsigned long long* next, int* err)
 {
   constexpr int kSlots = kWarps / kPoiWarps;
@@ -2923,7 +2963,7 @@ __global__ void __launch_bounds__(kWarps * 32, icgn_min_blocks(kWarps))
 // k_icgn_pair_px's windows (each job's map in device memory, win_bytes the window of the
 // launch's largest radius).  kMode 2: TMA windows (every job has a map), 0: no windows.
 template <int kPoiWarps, int kWarps, int kMode>
-__global__ void __launch_bounds__(kWarps * 32, pair_px_min_blocks(kWarps))
+__global__ void __launch_bounds__(kWarps * 32, px_min_blocks(kWarps))
     k_icgn_batch_pair_px(const BatchJob* __restrict__ jobs, int njobs, dic_poi* pois, const PoiRef* poi_ref,
                          int64_t begin, int64_t end, unsigned long long* next, float conv, float max_iter,
                          unsigned long long* iter_sum, uint32_t win_bytes, uint32_t wait_polls, int* err)
