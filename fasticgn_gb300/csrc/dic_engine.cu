@@ -239,13 +239,20 @@ struct dic_cnn
   X(34, 8, true) X(36, 8, false) X(38, 5, true) X(40, 4, false) X(42, 3, false) X(44, 5, false) X(46, 2, true) \
   X(48, 2, false) X(50, 3, false) X(52, 3, false) X(54, 1, false) X(56, 1, false) X(58, 1, true) X(60, 1, false) \
   X(62, 1, true) X(64, 1, false)
-constexpr unsigned kNearCtas = 608;   // CTAs of a second pass at most: near ties are rare
+// CTAs of a second pass, and of a pass behind a device switch, at most: near ties are rare, and
+// so are the frames that switch a repair pass on
+constexpr unsigned kFewCtas = 1216;
+unsigned fftcc_grid(const FftccParams& p, int per_cta)
+{
+  const int64_t blocks = (p.n + per_cta - 1) / per_cta;
+  return (unsigned)(p.enable ? std::min<int64_t>(blocks, kFewCtas) : blocks);
+}
 template <int M, int kPois, bool kPrime>
 void launch_fftcc_line(const FftccParams& p, cudaStream_t st)
 {
   using F = FftccLine<M, kPois>;
-  k_fftcc_line<M, kPois><<<(unsigned)((p.n + kPois - 1) / kPois), F::kThreads, F::kSmem, st>>>(p);
-  const unsigned second = (unsigned)std::min<int64_t>(p.n, kNearCtas);
+  k_fftcc_line<M, kPois><<<fftcc_grid(p, kPois), F::kThreads, F::kSmem, st>>>(p);
+  const unsigned second = (unsigned)std::min<int64_t>(p.n, kFewCtas);
   if constexpr (kPrime)
     k_fftcc_large<<<second, 256, (size_t)2 * M * (M + 1) * sizeof(float2), st>>>(p, M);
   else
@@ -254,9 +261,9 @@ void launch_fftcc_line(const FftccParams& p, cudaStream_t st)
 template <int M>
 void launch_fftcc2(const FftccParams& p, cudaStream_t st)
 {
-  const unsigned blocks = (unsigned)((p.n + 3) / 4);
+  const unsigned blocks = fftcc_grid(p, 4);
   k_fftcc2<M><<<blocks, 64, 0, st>>>(p);
-  if constexpr (fftcc2_near(M)) k_fftcc2<M, true><<<std::min(blocks, kNearCtas), 64, 0, st>>>(p);
+  if constexpr (fftcc2_near(M)) k_fftcc2<M, true><<<std::min(blocks, kFewCtas), 64, 0, st>>>(p);
 }
 // whether a length's launch fills a list of near ties (FftccParams::near)
 bool fftcc_near(int m) { return m > 32 || (m >= 8 && m <= 30 && fftcc2_near(m)); }

@@ -3499,9 +3499,9 @@ __host__ __device__ constexpr bool fftcc2_near(int m)
   return false;
 }
 // Two POIs on the calling warp: queue indices i0, i0 + 1, or (kSecond) the entries i0, i0 + 1 of
-// P.near, of which `listed` exist; zs: the warp's two windows.
+// P.near, of which `count` exist; zs: the warp's two windows.
 template <int M, bool kSecond>
-__device__ __forceinline__ void fftcc2_warp(const FftccParams& P, int64_t i0, int64_t listed, float2* zs)
+__device__ __forceinline__ void fftcc2_warp(const FftccParams& P, int64_t i0, int64_t count, float2* zs)
 {
   static_assert(M % 2 == 0 && M / 2 + 1 <= 16, "16 inverse lanes per POI");
   constexpr int R = M / 2, S = M + 1;
@@ -3519,9 +3519,8 @@ __device__ __forceinline__ void fftcc2_warp(const FftccParams& P, int64_t i0, in
 #pragma unroll 1
   for (int q = 0; q < 2; ++q)
   {
-    const bool in = !kSecond || i0 + q < listed;
-    const int64_t i = in ? index(q) : 0;
-    bool lv = in && queue_slot_active(P, i);
+    bool lv = i0 + q < count;
+    const int64_t i = lv ? index(q) : 0;
     float ui = 0.f, vi = 0.f, px = 0.f, py = 0.f;
     if (lv)
     {
@@ -3708,6 +3707,18 @@ __device__ __forceinline__ void fftcc2_warp(const FftccParams& P, int64_t i0, in
   }
 }
 
+// entries a launch has to go through: the queue, or (kSecond) the list
+template <bool kSecond>
+__device__ __forceinline__ int64_t fftcc_count(const FftccParams& P)
+{
+  if constexpr (kSecond) return (int64_t)*P.near_n;
+  if (P.enable && *P.enable == 0) return 0;
+  return P.n_dev ? *P.n_dev : P.n;
+}
+
+// The grid covers the queue, or is a few CTAs per SM that go on through it: a launch behind a
+// device switch that is off (a stream's repair passes, almost always) then costs 6 us where the
+// full grid's empty CTAs took 34 (162 000 POIs).
 template <int M, bool kSecond = false>
 // (Register caps for 7 or 8 CTAs per SM spill: 0.93 against 0.67 ms at 2048^2.)
 __global__ void __launch_bounds__(64) k_fftcc2(FftccParams P)
@@ -3715,18 +3726,12 @@ __global__ void __launch_bounds__(64) k_fftcc2(FftccParams P)
   constexpr int kWarps = 2, S = M + 1;
   __shared__ float2 smem[kWarps * 2][M * S];
   const int warp = threadIdx.x >> 5;
-  const int64_t first = ((int64_t)blockIdx.x * kWarps + warp) * 2;
-  if constexpr (kSecond)
+  const int64_t count = fftcc_count<kSecond>(P);
+  for (int64_t k = ((int64_t)blockIdx.x * kWarps + warp) * 2; k < count; k += (int64_t)gridDim.x * kWarps * 2)
   {
-    const int64_t listed = (int64_t)*P.near_n;
-    for (int64_t k = first; k < listed; k += (int64_t)gridDim.x * kWarps * 2)
-    {
-      fftcc2_warp<M, true>(P, k, listed, smem[warp * 2]);
-      __syncwarp();
-    }
+    fftcc2_warp<M, kSecond>(P, k, count, smem[warp * 2]);
+    __syncwarp();
   }
-  else
-    fftcc2_warp<M, false>(P, first, 0, smem[warp * 2]);
 }
 
 // --------------------------------------------------------------------------------------
@@ -4328,8 +4333,9 @@ struct FftccLine
   static constexpr int kThreads = (kPois * M + 31) / 32 * 32;
   static constexpr size_t kSmem = (size_t)kPois * M * (M + 1) * sizeof(float2);
 };
+// POIs base .. base + kPois - 1 of the queue, of which those below count exist
 template <int M, int kPois>
-__global__ void __launch_bounds__(FftccLine<M, kPois>::kThreads) k_fftcc_line(FftccParams P)
+__device__ __forceinline__ void fftcc_line_block(const FftccParams& P, int64_t base, int64_t count)
 {
   using L = LinePlan<M>;
   constexpr int S = L::S, R = L::R, kThreads = FftccLine<M, kPois>::kThreads;
@@ -4340,11 +4346,10 @@ __global__ void __launch_bounds__(FftccLine<M, kPois>::kThreads) k_fftcc_line(Ff
   const int tid = threadIdx.x;
   const int w = P.w, h = P.h;
   const int q = tid / M, c = tid % M;
-  const int64_t i = (int64_t)blockIdx.x * kPois + q;
-  if (!queue_slot_active(P, (int64_t)blockIdx.x * kPois)) return;   // the whole CTA
+  const int64_t i = base + q;
   // a POI's threads decide alike; out-of-range POIs are left untouched, as the CPU leaves them
   float px = 0.f, py = 0.f, ui = 0.f, vi = 0.f;
-  bool on = q < kPois && queue_slot_active(P, i);
+  bool on = q < kPois && i < count;
   if (on)
   {
     const dic_poi* poi = P.pois + i;
@@ -4499,6 +4504,18 @@ __global__ void __launch_bounds__(FftccLine<M, kPois>::kThreads) k_fftcc_line(Ff
     poi->u0 = ui;
     poi->v0 = vi;
     poi->zncc = top / (sqrtf(norm.x * norm.y) * (float)(M * M));
+  }
+}
+
+// grid as k_fftcc2's
+template <int M, int kPois>
+__global__ void __launch_bounds__(FftccLine<M, kPois>::kThreads) k_fftcc_line(FftccParams P)
+{
+  const int64_t count = fftcc_count<false>(P);
+  for (int64_t base = (int64_t)blockIdx.x * kPois; base < count; base += (int64_t)gridDim.x * kPois)
+  {
+    fftcc_line_block<M, kPois>(P, base, count);
+    __syncthreads();
   }
 }
 
