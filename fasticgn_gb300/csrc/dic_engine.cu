@@ -409,18 +409,14 @@ struct dic_engine
   template <typename T>
   void launch_prepare_ref()
   {
-    dim3 grid((w + kPrepTile - 1) / kPrepTile, (h + kPrepTile - 1) / kPrepTile);
-    k_prepare_ref<T><<<grid, 256, 0, stream>>>(reinterpret_cast<const T*>(raw_ref.ptr), w, h, scale(),
-                                               ref_f32.ptr, ref_pack.ptr);
+    launch_ref_planes(reinterpret_cast<const T*>(raw_ref.ptr), w, h, scale(), ref_f32.ptr, ref_pack.ptr, stream);
     check_launch("k_prepare_ref");
   }
   template <typename T>
   void launch_prepare_tar(bool table, bool pitched)
   {
-    dim3 grid((w + kPrepTile - 1) / kPrepTile, (h + kPrepTile - 1) / kPrepTile);
-    k_prepare_tar<T><<<grid, 256, 0, stream>>>(reinterpret_cast<const T*>(raw_tar.ptr), w, h, scale(),
-                                               tar_f32.ptr, table ? coef.ptr : nullptr, lattice.ptr,
-                                               pitched ? tar_px.ptr : nullptr, px_pitch(w));
+    launch_tar_planes(reinterpret_cast<const T*>(raw_tar.ptr), w, h, scale(), tar_f32.ptr, table ? coef.ptr : nullptr,
+                      lattice.ptr, pitched ? tar_px.ptr : nullptr, px_pitch(w), stream);
     check_launch("k_prepare_tar");
   }
 
@@ -1779,13 +1775,10 @@ struct dic_engine
   void prep_planes(const unsigned char* raw_r, const unsigned char* raw_t, int bw, int bh, JobBufs& J, bool table,
                    bool pitched, cudaStream_t st)
   {
-    dim3 grid((bw + kPrepTile - 1) / kPrepTile, (bh + kPrepTile - 1) / kPrepTile);
-    k_prepare_ref<T><<<grid, 256, 0, st>>>(reinterpret_cast<const T*>(raw_r), bw, bh, scale(), J.ref_f32.ptr,
-                                               J.ref_pack.ptr);
+    launch_ref_planes(reinterpret_cast<const T*>(raw_r), bw, bh, scale(), J.ref_f32.ptr, J.ref_pack.ptr, st);
     check_launch("k_prepare_ref");
-    k_prepare_tar<T><<<grid, 256, 0, st>>>(reinterpret_cast<const T*>(raw_t), bw, bh, scale(), J.tar_f32.ptr,
-                                           table ? J.coef.ptr : nullptr, J.lattice.ptr,
-                                           pitched ? J.tar_px.ptr : nullptr, px_pitch(bw));
+    launch_tar_planes(reinterpret_cast<const T*>(raw_t), bw, bh, scale(), J.tar_f32.ptr, table ? J.coef.ptr : nullptr,
+                      J.lattice.ptr, pitched ? J.tar_px.ptr : nullptr, px_pitch(bw), st);
     check_launch("k_prepare_tar");
   }
 
@@ -3332,9 +3325,8 @@ template <typename T>
 void noalloc_prepare(const void* ref, const void* tar, int w, int h, float scale, float* ref_f32,
                      float4* ref_pack, float* tar_f32, float4* coef, cudaStream_t s)
 {
-  dim3 grid((w + kPrepTile - 1) / kPrepTile, (h + kPrepTile - 1) / kPrepTile);
-  k_prepare_ref<T><<<grid, 256, 0, s>>>(static_cast<const T*>(ref), w, h, scale, ref_f32, ref_pack);
-  k_prepare_tar<T><<<grid, 256, 0, s>>>(static_cast<const T*>(tar), w, h, scale, tar_f32, coef);
+  launch_ref_planes(static_cast<const T*>(ref), w, h, scale, ref_f32, ref_pack, s);
+  launch_tar_planes<T>(static_cast<const T*>(tar), w, h, scale, tar_f32, coef, nullptr, nullptr, 0, s);
 }
 }  // namespace
 

@@ -98,55 +98,106 @@ __device__ __forceinline__ float load_px<float>(const float* p, size_t i, float 
 
 // --------------------------------------------------------------------------------------
 // Reference prep: raw -> float plane, Gradient2D4 (src/oc_gradient.cpp:37-79), packed
-// {ref, gx, gy, 0}.  16x16 output tile per 256-thread block, 2-px halo staged in smem.
+// {ref, gx, gy, 0}.  64x16 output tile per 256-thread block, 2-px halo staged in smem; a thread
+// takes one column of four rows, whose vertical neighbours it reads once.
 // Stencil term order follows the CPU: -f(c+2)/12 + 2f(c+1)/3 - 2f(c-1)/3 + f(c-2)/12,
 // each product rounded separately (no contraction), so planes are bit-identical.
+// Bound by its writes (20 B a pixel: 84 MB at 2048^2).  With 16x16 tiles, one pixel per thread,
+// the halo (400 loads for 256 pixels) and the short blocks took longer than the writes:
+// 2048^2 uint8 28 -> 18 us.
 // --------------------------------------------------------------------------------------
-constexpr int kPrepTile = 16;
+constexpr int kPrepTile = 16;   // k_prepare_tar
+constexpr int kRefTileW = 64, kRefTileH = 16, kRefRows = 4;
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_prepare_ref(const T* __restrict__ raw, int w, int h, float scale,
                                                      float* __restrict__ ref_f32,
                                                      float4* __restrict__ ref_pack)
 {
-  __shared__ float tile[kPrepTile + 4][kPrepTile + 4 + 1];
-  const int bx = blockIdx.x * kPrepTile, by = blockIdx.y * kPrepTile;
-  for (int i = threadIdx.x; i < (kPrepTile + 4) * (kPrepTile + 4); i += blockDim.x)
+  constexpr int kW = kRefTileW + 4, kH = kRefTileH + 4;
+  __shared__ float tile[kH][kW];
+  const int bx = blockIdx.x * kRefTileW, by = blockIdx.y * kRefTileH;
+  for (int i = threadIdx.x; i < kW * kH; i += 256)
   {
-    int ty = i / (kPrepTile + 4), tx = i % (kPrepTile + 4);
-    int gx = bx + tx - 2, gy = by + ty - 2;
+    const int ty = i / kW, tx = i % kW;
+    const int gx = bx + tx - 2, gy = by + ty - 2;
     float v = 0.f;
     if (gx >= 0 && gx < w && gy >= 0 && gy < h) v = load_px<T>(raw, (size_t)gy * w + gx, scale);
     tile[ty][tx] = v;
   }
   __syncthreads();
-  const int tx = threadIdx.x % kPrepTile, ty = threadIdx.x / kPrepTile;
-  const int x = bx + tx, y = by + ty;
-  if (x >= w || y >= h) return;
-  const float c = tile[ty + 2][tx + 2];
+  const int tx = threadIdx.x % kRefTileW, ty = threadIdx.x / kRefTileW * kRefRows;
+  const int x = bx + tx;
+  if (x >= w) return;
   const float f1 = 1.f / 12.f, f2 = 2.f / 3.f;
-  float gxv = 0.f, gyv = 0.f;
-  if (x >= 2 && x < w - 2)
+  const bool inx = x >= 2 && x < w - 2;
+  float v[kRefRows + 4];
+#pragma unroll
+  for (int k = 0; k < kRefRows + 4; ++k) v[k] = tile[ty + k][tx + 2];
+#pragma unroll
+  for (int k = 0; k < kRefRows; ++k)
   {
-    float r = 0.f;
-    r = __fsub_rn(r, __fmul_rn(tile[ty + 2][tx + 4], f1));
-    r = __fadd_rn(r, __fmul_rn(tile[ty + 2][tx + 3], f2));
-    r = __fsub_rn(r, __fmul_rn(tile[ty + 2][tx + 1], f2));
-    r = __fadd_rn(r, __fmul_rn(tile[ty + 2][tx + 0], f1));
-    gxv = r;
+    const int y = by + ty + k;
+    if (y >= h) return;
+    float gxv = 0.f, gyv = 0.f;
+    if (inx)
+    {
+      float r = 0.f;
+      r = __fsub_rn(r, __fmul_rn(tile[ty + k + 2][tx + 4], f1));
+      r = __fadd_rn(r, __fmul_rn(tile[ty + k + 2][tx + 3], f2));
+      r = __fsub_rn(r, __fmul_rn(tile[ty + k + 2][tx + 1], f2));
+      r = __fadd_rn(r, __fmul_rn(tile[ty + k + 2][tx + 0], f1));
+      gxv = r;
+    }
+    if (y >= 2 && y < h - 2)
+    {
+      float r = 0.f;
+      r = __fsub_rn(r, __fmul_rn(v[k + 4], f1));
+      r = __fadd_rn(r, __fmul_rn(v[k + 3], f2));
+      r = __fsub_rn(r, __fmul_rn(v[k + 1], f2));
+      r = __fadd_rn(r, __fmul_rn(v[k], f1));
+      gyv = r;
+    }
+    const size_t o = (size_t)y * w + x;
+    ref_f32[o] = v[k + 2];
+    ref_pack[o] = make_float4(v[k + 2], gxv, gyv, 0.f);
   }
-  if (y >= 2 && y < h - 2)
-  {
-    float r = 0.f;
-    r = __fsub_rn(r, __fmul_rn(tile[ty + 4][tx + 2], f1));
-    r = __fadd_rn(r, __fmul_rn(tile[ty + 3][tx + 2], f2));
-    r = __fsub_rn(r, __fmul_rn(tile[ty + 1][tx + 2], f2));
-    r = __fadd_rn(r, __fmul_rn(tile[ty + 0][tx + 2], f1));
-    gyv = r;
-  }
-  const size_t o = (size_t)y * w + x;
-  ref_f32[o] = c;
-  ref_pack[o] = make_float4(c, gxv, gyv, 0.f);
+}
+
+template <typename T>
+void launch_ref_planes(const T* raw, int w, int h, float scale, float* ref_f32, float4* ref_pack, cudaStream_t st)
+{
+  const dim3 grid((w + kRefTileW - 1) / kRefTileW, (h + kRefTileH - 1) / kRefTileH);
+  k_prepare_ref<T><<<grid, 256, 0, st>>>(raw, w, h, scale, ref_f32, ref_pack);
+}
+
+// --------------------------------------------------------------------------------------
+// Target plane alone, for pixel sampling: raw -> float, and (tar_px, nullable) again with rows
+// of `pitch` floats (a multiple of 4), for the TMA windows when W itself is not a multiple of
+// 4.  A thread takes one column of four rows, so four loads are in flight and any W and any
+// alignment of `raw` will do.  k_prepare_tar without its table went through its 19x19 halo
+// tiles for this: 2048^2 uint16 27 -> 6.6 us, 1024^2 uint8 8.0 -> 2.9.  The grid is linear (row blocks x column blocks), so any H will do as well.
+// --------------------------------------------------------------------------------------
+constexpr int kPlaneThreads = 128, kPlaneRows = 4;
+template <typename T>
+__global__ void __launch_bounds__(kPlaneThreads) k_target_plane(const T* __restrict__ raw, int w, int h, float scale,
+                                                                float* __restrict__ tar_f32,
+                                                                float* __restrict__ tar_px, int pitch)
+{
+  const unsigned across = (unsigned)((w - 1) / kPlaneThreads + 1), by = blockIdx.x / across;
+  const int x = (int)(blockIdx.x - by * across) * kPlaneThreads + (int)threadIdx.x, y0 = (int)by * kPlaneRows;
+  if (x >= w) return;
+  float v[kPlaneRows];
+#pragma unroll
+  for (int k = 0; k < kPlaneRows; ++k)
+    if (y0 + k < h) v[k] = load_px<T>(raw, (size_t)(y0 + k) * w + x, scale);
+#pragma unroll
+  for (int k = 0; k < kPlaneRows; ++k)
+    if (y0 + k < h)
+    {
+      tar_f32[(size_t)(y0 + k) * w + x] = v[k];
+      if (tar_px) tar_px[(size_t)(y0 + k) * pitch + x] = v[k];
+    }
 }
 
 // --------------------------------------------------------------------------------------
@@ -161,8 +212,7 @@ __global__ void __launch_bounds__(256) k_prepare_ref(const T* __restrict__ raw, 
 // IC-GN time on GB300, same values (the texel-major 64 B layout spreads a warp load over
 // 16 cache lines).
 // --------------------------------------------------------------------------------------
-// tar_px (nullable): the float plane again with rows of `pitch` floats (a multiple of 4), for
-// the pixel-sampled IC-GN's TMA windows when W itself is not a multiple of 4.
+// tar_px (nullable): as k_target_plane's.
 template <typename T>
 __global__ void __launch_bounds__(256) k_prepare_tar(const T* __restrict__ raw, int w, int h, float scale,
                                                      float* __restrict__ tar_f32,
@@ -186,7 +236,6 @@ __global__ void __launch_bounds__(256) k_prepare_tar(const T* __restrict__ raw, 
   const size_t o = (size_t)y * w + x;
   tar_f32[o] = tile[ty + 1][tx + 1];
   if (tar_px) tar_px[(size_t)y * pitch + x] = tile[ty + 1][tx + 1];
-  if (!coef) return;   // pixel sampling: no table
   const size_t plane = (size_t)w * h;
   float4* dst = coef + 2 * o;   // row k at dst[(k >> 1) * 2 * plane + (k & 1)]
   if (x < 1 || y < 1 || x >= w - 2 || y >= h - 2)
@@ -220,6 +269,21 @@ __global__ void __launch_bounds__(256) k_prepare_tar(const T* __restrict__ raw, 
     dst[(k >> 1) * 2 * plane + (k & 1)] = make_float4(p[3 - k][3], p[3 - k][2], p[3 - k][1], p[3 - k][0]);
   // the interpolant at the texel's own integer position (dx = dy = 0): coefficient [0][0]
   if (lattice) lattice[o] = p[3][3];
+}
+
+// the target's planes: with the table (coef) or, for pixel sampling, without
+template <typename T>
+void launch_tar_planes(const T* raw, int w, int h, float scale, float* tar_f32, float4* coef, float* lattice,
+                       float* tar_px, int pitch, cudaStream_t st)
+{
+  if (!coef)
+  {
+    const unsigned blocks = (unsigned)((w - 1) / kPlaneThreads + 1) * (unsigned)((h - 1) / kPlaneRows + 1);
+    k_target_plane<T><<<blocks, kPlaneThreads, 0, st>>>(raw, w, h, scale, tar_f32, tar_px, pitch);
+    return;
+  }
+  const dim3 grid((w + kPrepTile - 1) / kPrepTile, (h + kPrepTile - 1) / kPrepTile);
+  k_prepare_tar<T><<<grid, 256, 0, st>>>(raw, w, h, scale, tar_f32, coef, lattice, tar_px, pitch);
 }
 
 // --------------------------------------------------------------------------------------
