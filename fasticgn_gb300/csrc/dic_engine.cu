@@ -556,9 +556,14 @@ struct dic_engine
     if (n > 0)
     {
       mark(kPhPoi, 0);
-      const unsigned blocks = (unsigned)((n + kPrepPois - 1) / kPrepPois);
-      k_poi_prepare32<<<blocks, kPrepWarps * 32, 0, stream>>>(ref_pack.ptr, w, h, src, n, cfg.subset_radius_x,
-                                                              cfg.subset_radius_y, poi_ref.ptr);
+      int sms = 0;
+      DIC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg.device));
+      if (n <= (int64_t)kPrepFewPerSm * sms)
+        k_poi_prepare32<kPrepPoisFew><<<(unsigned)((n + kPrepPoisFew - 1) / kPrepPoisFew), kPrepWarps * 32, 0, stream>>>(
+            ref_pack.ptr, w, h, src, n, cfg.subset_radius_x, cfg.subset_radius_y, poi_ref.ptr);
+      else
+        k_poi_prepare32<kPrepPois><<<(unsigned)((n + kPrepPois - 1) / kPrepPois), kPrepWarps * 32, 0, stream>>>(
+            ref_pack.ptr, w, h, src, n, cfg.subset_radius_x, cfg.subset_radius_y, poi_ref.ptr);
       check_launch("k_poi_prepare32");
       mark(kPhPoi, 1);
     }
@@ -1974,7 +1979,7 @@ struct dic_engine
       const int r = J.subset_radius;
       dic_poi* q = bq.ptr + b_first[k];
       DIC_CUDA(cudaMemcpyAsync(q, J.pois, sizeof(dic_poi) * J.count, in_kind, st));
-      k_poi_prepare32<<<(unsigned)((J.count + kPrepPois - 1) / kPrepPois), kPrepWarps * 32, 0, st>>>(
+      k_poi_prepare32<kPrepPois><<<(unsigned)((J.count + kPrepPois - 1) / kPrepPois), kPrepWarps * 32, 0, st>>>(
           M.ref_pack.ptr, J.width, J.height, q, J.count, r, r, bpoi.ptr + b_first[k]);
       check_launch("k_poi_prepare32");
       FftccParams fp{M.ref_f32.ptr, M.tar_f32.ptr, q, J.count, J.width, J.height};

@@ -773,23 +773,30 @@ __global__ void __launch_bounds__(128) k_poi_prepare(const float4* __restrict__ 
 // 171 024 POIs at r 7: 0.24 -> 0.18; r 20, 29 000 POIs: 0.166 -> 0.094; r 30: 0.23 -> 0.20.
 // --------------------------------------------------------------------------------------
 constexpr int kPrepPois = 32, kPrepWarps = 4;   // (8 warps per 32 POIs: 0.72 against 0.60 ms at 2048^2)
+// A queue of at most kPrepFewPerSm POIs per SM (three CTAs of 32, half of what fits) leaves SMs
+// idle while each warp takes its eight POIs one after the other: it gets eight POIs per CTA, two
+// per warp.  2300 POIs, r 15: 51 -> 18 us; 12 600, r 31: 96 -> 67; above the line 29 000, r 20
+// would go 94 -> 111, since columns are then formed by more CTAs.  A batch's jobs fill the SMs
+// for one another and keep 32 (5.65 against 5.68 ms for eight uneven jobs).
+constexpr int kPrepPoisFew = 8, kPrepFewPerSm = 96;
 constexpr int kPrepCols = 256;   // shared columns per grid row (32 POIs at step <= 7 for r 15, <= 6 for r 30)
 #ifndef DIC_PREP_SHARED_COLUMNS
 #define DIC_PREP_SHARED_COLUMNS 1
 #endif
+template <int kPois>
 __global__ void __launch_bounds__(kPrepWarps * 32, 6) k_poi_prepare32(const float4* __restrict__ ref_pack, int w,
                                                                   int h, const dic_poi* __restrict__ pois,
                                                                   int64_t n, int rx, int ry,
                                                                   PoiRef* __restrict__ out)
 {
-  __shared__ float sh_h[kPrepPois * 21];       // odd stride: lane p reads row p conflict-free
-  __shared__ float sh_inv[kPrepPois * 37];
-  __shared__ int sh_live[kPrepPois];
+  __shared__ float sh_h[kPois * 21];       // odd stride: lane p reads row p conflict-free
+  __shared__ float sh_inv[kPois * 37];
+  __shared__ int sh_live[kPois];
   __shared__ float sh_col[2][kColSums][kPrepCols];
   __shared__ int sh_row[2][3];                 // per grid row: cy, first column, columns
   __shared__ int sh_shared;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t base = (int64_t)blockIdx.x * kPrepPois;
+  const int64_t base = (int64_t)blockIdx.x * kPois;
   const int size = (2 * rx + 1) * (2 * ry + 1);
   if (warp == 0)
   {
@@ -797,7 +804,7 @@ __global__ void __launch_bounds__(kPrepWarps * 32, 6) k_poi_prepare32(const floa
     const int64_t i = base + lane;
     bool valid = false;
     int pcx = 0, pcy = 0;
-    if (i < n)
+    if (lane < kPois && i < n)
     {
       const float px = pois[i].x, py = pois[i].y;
       valid = py - ry >= 0 && px - rx >= 0 && py + ry <= h - 1 && px + rx <= w - 1;
@@ -844,7 +851,7 @@ __global__ void __launch_bounds__(kPrepWarps * 32, 6) k_poi_prepare32(const floa
     }
     __syncthreads();
   }
-  for (int k = 0; k < kPrepPois / kPrepWarps; ++k)
+  for (int k = 0; k < kPois / kPrepWarps; ++k)
   {
     const int p = warp + kPrepWarps * k;
     const int64_t i = base + p;
@@ -869,7 +876,7 @@ __global__ void __launch_bounds__(kPrepWarps * 32, 6) k_poi_prepare32(const floa
     if (lane == 0) sh_live[p] = live ? 1 : 0;
   }
   __syncthreads();
-  if (warp == 0 && sh_live[lane])
+  if (warp == 0 && lane < kPois && sh_live[lane])
   {
     float hf[6][6];
     int t = 0;
@@ -894,7 +901,7 @@ __global__ void __launch_bounds__(kPrepWarps * 32, 6) k_poi_prepare32(const floa
     }
   }
   __syncthreads();
-  for (int idx = threadIdx.x; idx < kPrepPois * 36; idx += kPrepWarps * 32)
+  for (int idx = threadIdx.x; idx < kPois * 36; idx += kPrepWarps * 32)
   {
     const int p = idx / 36, e = idx - p * 36;
     if (sh_live[p]) out[base + p].inv_h[e] = sh_inv[p * 37 + e];
