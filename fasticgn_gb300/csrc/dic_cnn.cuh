@@ -178,7 +178,7 @@ __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float
 // other layers use mma.sync.  One 512-thread CTA per SM holds two independent warp groups
 // of 8 warps; each group runs tiles of kT = 2 POIs (tiles strided over groups and CTAs) and
 // syncs on its own named barrier, so one group's serial phases (window staging, conv3/conv4,
-// the MLP) overlap the other's conv1/conv2.  Same arithmetic as the GEMM path (BF16
+// the MLP) overlap the other's conv1/conv2.  Same arithmetic as the training layers (BF16
 // operands, FP32 accumulation, BF16 ReLU outputs), so both give the same seeds up to
 // accumulation order.
 //

@@ -262,7 +262,8 @@ template <int M>
 void launch_fftcc2(const FftccParams& p, cudaStream_t st)
 {
   const unsigned blocks = fftcc_grid(p, 4);
-  k_fftcc2<M><<<blocks, 64, 0, st>>>(p);
+  if (p.enable) k_fftcc2<M, false, true><<<blocks, 64, 0, st>>>(p);
+  else k_fftcc2<M><<<blocks, 64, 0, st>>>(p);
   if constexpr (fftcc2_near(M)) k_fftcc2<M, true><<<std::min(blocks, kFewCtas), 64, 0, st>>>(p);
 }
 // whether a length's launch fills a list of near ties (FftccParams::near)
@@ -707,8 +708,8 @@ struct dic_engine
   // four-plane table); the autotuner still times both forms.  shape[0]: single queues,
   // shape[1]: batches.
   // The pixel pair walk's default (2 warps per CTA, 2 per POI, TMA windows) is its fastest
-  // measured form on the 2048² pair at r 20 and 30 (5.84 and 8.05 ms; 4 warps per CTA 7.15 and
-  // 11.8, 8 warps 7.16 and 12.6, one warp per POI 6.9 and 17.1).
+  // measured form on the 2048² pair at r 20 and 30 (with the ungrouped row loop 5.84 and 8.05 ms; 4 warps per
+  // CTA 7.15 and 11.8, 8 warps 7.16 and 12.6, one warp per POI 6.9 and 17.1).
   IcgnShape shape[2][kWalks] = {{{4, 8, 0.f}, {4, 8, 0.f}, {4, 8, 0.f}, {4, 0, 0.f, 1}, {2, 0, 0.f, 1, 2}},
                                 {{4, 7, 0.f}, {4, 7, 0.f}, {4, 7, 0.f}, {4, 0, 0.f}, {2, 0, 0.f, 0, 2}}};
   bool tuned[2][kWalks] = {};

@@ -1199,9 +1199,9 @@ __device__ __forceinline__ float pixel_at(const PixelTile& T, const float* __res
 // not all inside the range and the window: per-sample range tests, window or global-plane
 // reads, the same sums in the same order as the fast loop.  Returns the sums (A0, A1, A2, B0,
 // B2, B3, B5) and whether a sample left the range.  (The fast loop's code generation is
-// sensitive to this rare path: written as this function and inlined, k_icgn_px runs 2.80 ms
-// on the 2048x2048 pair; as a call, 2.84 ms; as the same loop written inside icgn_solve with
-// the padded pitch, 3.00 ms.)
+// sensitive to this rare path: with the ungrouped row loop k_icgn_px ran 2.80 ms of full
+// iterations on the 2048x2048 pair written as this function and inlined, 2.84 ms as a call, 3.00 ms
+// as the same loop inside the solver with the padded pitch.)
 struct ColumnSums
 {
   float A0, A1, A2, B0, B2, B3, B5;
@@ -3590,8 +3590,9 @@ __device__ __forceinline__ void fftcc2_warp(const FftccParams& P, int64_t i0, in
 #pragma unroll 1
   for (int q = 0; q < 2; ++q)
   {
-    bool lv = i0 + q < count;
-    const int64_t i = lv ? index(q) : 0;
+    const bool in = !kSecond || i0 + q < count;
+    const int64_t i = in ? index(q) : 0;
+    bool lv = in && queue_slot_active(P, i);
     float ui = 0.f, vi = 0.f, px = 0.f, py = 0.f;
     if (lv)
     {
@@ -3787,22 +3788,29 @@ __device__ __forceinline__ int64_t fftcc_count(const FftccParams& P)
   return P.n_dev ? *P.n_dev : P.n;
 }
 
-// The grid covers the queue, or is a few CTAs per SM that go on through it: a launch behind a
-// device switch that is off (a stream's repair passes, almost always) then costs 6 us where the
-// full grid's empty CTAs took 34 (162 000 POIs).
-template <int M, bool kSecond = false>
+// The grid covers the queue, or (kWalk) is a few CTAs per SM that go on through it: a launch behind
+// a device switch that is off (a stream's repair passes, almost always) then costs 6 us where the
+// full grid's empty CTAs took 34 (162 000 POIs).  The loop costs the transforms their schedule
+// (k_fftcc2<30> 0.65 against 0.61 ms at 2048^2), so launches without a switch go without it.
+template <int M, bool kSecond = false, bool kWalk = kSecond>
 // (Register caps for 7 or 8 CTAs per SM spill: 0.93 against 0.67 ms at 2048^2.)
 __global__ void __launch_bounds__(64) k_fftcc2(FftccParams P)
 {
   constexpr int kWarps = 2, S = M + 1;
   __shared__ float2 smem[kWarps * 2][M * S];
   const int warp = threadIdx.x >> 5;
-  const int64_t count = fftcc_count<kSecond>(P);
-  for (int64_t k = ((int64_t)blockIdx.x * kWarps + warp) * 2; k < count; k += (int64_t)gridDim.x * kWarps * 2)
+  const int64_t first = ((int64_t)blockIdx.x * kWarps + warp) * 2;
+  if constexpr (kWalk)
   {
-    fftcc2_warp<M, kSecond>(P, k, count, smem[warp * 2]);
-    __syncwarp();
+    const int64_t count = fftcc_count<kSecond>(P);
+    for (int64_t k = first; k < count; k += (int64_t)gridDim.x * kWarps * 2)
+    {
+      fftcc2_warp<M, kSecond>(P, k, count, smem[warp * 2]);
+      __syncwarp();
+    }
   }
+  else
+    fftcc2_warp<M, false>(P, first, 0, smem[warp * 2]);
 }
 
 // --------------------------------------------------------------------------------------
@@ -3998,8 +4006,8 @@ __global__ void __launch_bounds__(256) k_fftcc_large(FftccParams P, int m)
 }
 
 // --------------------------------------------------------------------------------------
-// FFTCC for 32 < M <= 64 (subset radius 17..32) as a real FFT: one 128-thread CTA per POI,
-// the packed window z = ref + i tar in shared memory ([M][M + 1] float2; consecutive lanes
+// The second pass of 32 < M <= 64 where M is not 2 x prime: the near ties that k_fftcc_line lists,
+// in this kernel's own order of operations.  One 128-thread CTA per POI, the packed window z = ref + i tar in shared memory ([M][M + 1] float2; consecutive lanes
 // take consecutive lines, whose odd float2 stride keeps a warp's accesses conflict-free in
 // both directions), every line transform a four-step FFT M = N1 * N2 done in place by
 // small register FFTs:
