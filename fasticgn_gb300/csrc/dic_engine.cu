@@ -1521,6 +1521,23 @@ struct dic_engine
   bool use_graphs = true;
   cudaGraphExec_t seq_graph = nullptr;
   int seq_graph_kernels = 0;
+  // What a captured frame holds by value: the buffers its launches and copies name and the
+  // target's type.  Any other call on the engine may move one of them (a longer queue, a larger
+  // image), and a frame captured before that would replay on freed memory, so a replay compares
+  // this list with the one taken at the capture and captures again where they differ.
+  std::vector<const void*> seq_graph_args;
+  std::vector<const void*> frame_args() const
+  {
+    return {raw_tar.ptr, ref_f32.ptr, tar_f32.ptr, tar_px.ptr, ref_pack.ptr, coef.ptr, lattice.ptr, poi_ref.ptr,
+            queue.ptr, tmpl.ptr, prev.ptr, prev2.ptr, hist.ptr, scratch.ptr, fq.ptr, cand.ptr, fcount.ptr, baseline.ptr,
+            counters.ptr, icgn_next.ptr, wait_err.ptr, fft_near.ptr, fft_near_n.ptr,
+            reinterpret_cast<const void*>((uintptr_t)tar_dtype)};
+  }
+  void drop_seq_graph()
+  {
+    if (seq_graph) cudaGraphExecDestroy(seq_graph);
+    seq_graph = nullptr;
+  }
 
   void ensure_frame_buffers(int64_t n)
   {
@@ -2299,7 +2316,7 @@ void dic_engine_destroy(dic_engine* e)
   e->queue.release();
   e->slots.release();
   e->counters.release();
-  if (e->seq_graph) cudaGraphExecDestroy(e->seq_graph);
+  e->drop_seq_graph();
   e->drop_batch_graph();
   for (auto& ev : e->tune_ev)
     if (ev) cudaEventDestroy(ev);
@@ -2585,11 +2602,7 @@ int dic_sequence_begin(dic_engine* e, const dic_poi* pois, int64_t n, const dic_
       throw DicError{DIC_ERR_ARGUMENT, "FFTCC2D supports positive square radii only"};
     for (int64_t i = 0; i < n; ++i)
       if (!finite_xy(pois[i])) throw DicError{DIC_ERR_ARGUMENT, "sequence_begin: non-finite POI coordinate"};
-    if (e->seq_graph)
-    {
-      cudaGraphExecDestroy(e->seq_graph);
-      e->seq_graph = nullptr;
-    }
+    e->drop_seq_graph();
     e->ensure_frame_buffers(n);
     e->counters.ensure(1);
     DIC_CUDA(cudaMemcpyAsync(e->tmpl.ptr, pois, sizeof(dic_poi) * n, cudaMemcpyHostToDevice, e->stream));
@@ -2667,6 +2680,7 @@ int dic_sequence_frame(dic_engine* e, const void* px, int32_t w, int32_t h, int6
     }
     else if (e->use_graphs)
     {
+      if (e->seq_graph && e->frame_args() != e->seq_graph_args) e->drop_seq_graph();
       if (!e->seq_graph)
       {
         // Capture the steady-state frame once (all buffers exist after the first frame).
@@ -2698,6 +2712,7 @@ int dic_sequence_frame(dic_engine* e, const void* px, int32_t w, int32_t h, int6
           e->seq_graph = nullptr;
           throw DicError{DIC_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(ie)};
         }
+        e->seq_graph_args = e->frame_args();
       }
       DIC_CUDA(cudaGraphLaunch(e->seq_graph, e->stream));
       e->launches += e->seq_graph_kernels;
@@ -2754,11 +2769,7 @@ int dic_set_proposal(dic_engine* e, dic_cnn* net)
     if (net && net->device != e->cfg.device)
       throw DicError{DIC_ERR_ARGUMENT, "the proposal network lives on another device"};
     e->proposal = net;
-    if (e->seq_graph)
-    {
-      cudaGraphExecDestroy(e->seq_graph);   // it holds the previous network's weight pointers
-      e->seq_graph = nullptr;
-    }
+    e->drop_seq_graph();   // it holds the previous network's weight pointers
   });
 }
 
@@ -2879,12 +2890,7 @@ int dic_set_launch_shape(dic_engine* e, int32_t walk, const dic_launch_shape* sh
     }
     e->shape[0][walk] = sh;
     e->tuned[0][walk] = false;
-    if (e->seq_graph)
-    {
-      // a captured sequence frame holds the previous launch
-      cudaGraphExecDestroy(e->seq_graph);
-      e->seq_graph = nullptr;
-    }
+    e->drop_seq_graph();   // it holds the previous launch
   });
 }
 
@@ -2896,12 +2902,7 @@ int dic_set_sampling(dic_engine* e, int32_t mode)
     if (mode == e->sampling) return;
     e->sampling = mode;
     e->drop_batch_graph();   // a captured batch holds the previous kernels
-    if (e->seq_graph)
-    {
-      // a captured sequence frame holds the previous solver
-      cudaGraphExecDestroy(e->seq_graph);
-      e->seq_graph = nullptr;
-    }
+    e->drop_seq_graph();     // and so does a captured sequence frame
   });
 }
 
@@ -2909,13 +2910,9 @@ int dic_set_graphs(dic_engine* e, int32_t enabled)
 {
   return guarded(e, [&] {
     e->use_graphs = enabled != 0;
-    if (!e->use_graphs && e->seq_graph)
-    {
-      cudaGraphExecDestroy(e->seq_graph);
-      e->seq_graph = nullptr;
-    }
     if (!e->use_graphs)
     {
+      e->drop_seq_graph();
       e->drop_batch_graph();
       e->b_key_seen = false;
     }
