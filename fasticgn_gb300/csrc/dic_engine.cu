@@ -771,13 +771,16 @@ struct dic_engine
   }
   DevBuf<unsigned long long> icgn_next;   // work counter of the persistent single-queue launch
 
+  // k_icgn_px: dynamic shared memory of one CTA (its POIs' windows plus alignment room)
+  static size_t px_smem(int pois, int rx, int ry) { return 128 + (size_t)pois * px_window_bytes(rx, ry); }
   // Subsets of at most 16 columns take the form with two POIs per warp (k_icgn_px_half): one
-  // POI leaves half the lanes idle.
-  static int px_per_warp(int rx) { return 2 * rx + 1 <= kHalf ? 2 : 1; }
-  // k_icgn_px: dynamic shared memory of one CTA (the warps' windows plus alignment room)
-  static size_t px_smem(int warps, int rx, int ry)
+  // POI leaves half the lanes idle.  A tall subset's two windows per warp may not fit in a CTA
+  // where one does (8 warps from ry = 71 at rx = 7); it keeps one POI per warp.  While they fit,
+  // two are faster even at one CTA per SM: rx 7, ry 124, 9 744 POIs, 4 warps 1.23 against 1.64 ms.
+  int px_half_room = 0;   // dynamic shared memory a k_icgn_px_half CTA can have (px_attributes)
+  int px_per_warp(int warps, bool staged, int rx, int ry) const
   {
-    return 128 + (size_t)warps * px_per_warp(rx) * px_window_bytes(rx, ry);
+    return 2 * rx + 1 <= kHalf && (!staged || px_smem(2 * warps, rx, ry) <= (size_t)px_half_room) ? 2 : 1;
   }
   // the shared-memory opt-in of the three k_icgn_px widths (per engine, so per device): the
   // device's per-block maximum, set once outside any capture
@@ -804,6 +807,9 @@ struct dic_engine
     opt_in((const void*)k_icgn_px_half<2, 1>);
     opt_in((const void*)k_icgn_px_half<4, 1>);
     opt_in((const void*)k_icgn_px_half<8, 1>);
+    cudaFuncAttributes half{};
+    DIC_CUDA(cudaFuncGetAttributes(&half, (const void*)k_icgn_px_half<8, 2>));   // the largest static part
+    px_half_room = optin - (int)half.sharedSizeBytes;
     opt_in((const void*)k_icgn_batch_px<2, 2>);
     opt_in((const void*)k_icgn_batch_px<4, 2>);
     opt_in((const void*)k_icgn_batch_px<8, 2>);
@@ -824,9 +830,8 @@ struct dic_engine
     px_attr_set = true;
   }
   template <int W>
-  static int max_ctas_px(size_t smem, int rx)
+  static int max_ctas_px(size_t smem, bool two)
   {
-    const bool two = px_per_warp(rx) == 2;
     int b = 0;
     if (smem)
       DIC_CUDA(two ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_icgn_px_half<W, 2>, W * 32, smem)
@@ -858,8 +863,10 @@ struct dic_engine
     PxOcc& o = px_occ[slot];
     if (o.warps == warps && o.rx == rx && o.ry == ry) return o.ctas;
     px_attributes();
-    const size_t smem = staged ? px_smem(warps, rx, ry) : 0;
-    const int b = warps == 2 ? max_ctas_px<2>(smem, rx) : warps == 8 ? max_ctas_px<8>(smem, rx) : max_ctas_px<4>(smem, rx);
+    const int per = px_per_warp(warps, staged, rx, ry);
+    const size_t smem = staged ? px_smem(warps * per, rx, ry) : 0;
+    const bool two = per == 2;
+    const int b = warps == 2 ? max_ctas_px<2>(smem, two) : warps == 8 ? max_ctas_px<8>(smem, two) : max_ctas_px<4>(smem, two);
     if (b < 1) throw DicError{DIC_ERR_ARGUMENT, "IC-GN pixel windows of this subset radius do not fit in shared memory"};
     o = PxOcc{warps, staged ? 1 : 0, rx, ry, b};
     return b;
@@ -903,9 +910,9 @@ struct dic_engine
     DIC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg.device));
     const int warps = sh.warps;
     px_attributes();
-    const size_t smem = sh.tile ? px_smem(warps, p.rx, p.ry) : 0;
+    const int per = px_per_warp(warps, sh.tile != 0, p.rx, p.ry), per_cta = warps * per;
+    const size_t smem = sh.tile ? px_smem(per_cta, p.rx, p.ry) : 0;
     const int ctas = sh.ctas_per_sm > 0 ? sh.ctas_per_sm : occupancy_px(warps, sh.tile != 0, p.rx, p.ry);
-    const int per_cta = warps * px_per_warp(p.rx);
     const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)sms * ctas, (p.n + per_cta - 1) / per_cta));
     const CUtensorMap* m =
         sh.tile == 1 ? tar_map(p.tar, p.w, p.h, px_pitch(p.w), px_window_x(p.rx), px_window_y(p.ry)) : nullptr;
@@ -917,7 +924,7 @@ struct dic_engine
 #define DIC_PX_LAUNCH(W, M)                                                                                    \
   do                                                                                                              \
   {                                                                                                               \
-    if (px_per_warp(p.rx) == 2)                                                                                   \
+    if (per == 2)                                                                                                 \
       k_icgn_px_half<W, M><<<grid, W * 32, smem, stream>>>(q, m ? *m : none, icgn_next.ptr, wait_flag());         \
     else                                                                                                          \
       k_icgn_px<W, M><<<grid, W * 32, smem, stream>>>(q, m ? *m : none, icgn_next.ptr, wait_flag());              \
