@@ -1443,8 +1443,9 @@ __device__ __noinline__ ColumnSums px_column_lattice(int src, int pitch, const f
 }
 
 // One column's sums of an iteration: lane column flx under warp W, in the form the iteration
-// allows (covered: window_covers, lat: on_lattice, both warp-uniform).
-template <bool kPerRow = false>
+// allows (covered: window_covers, lat: on_lattice, both warp-uniform).  kWindow false: a kernel
+// without windows, where nothing is covered.
+template <bool kWindow, bool kPerRow = false>
 __device__ __forceinline__ ColumnSums px_column(const PixelTile& T, const float* __restrict__ tar,
                                                 const float4* __restrict__ ref_col, int w, int h, float px, float py,
                                                 const float (&W)[6], float flx, float t0, int ry, bool covered, bool lat,
@@ -1452,9 +1453,12 @@ __device__ __forceinline__ ColumnSums px_column(const PixelTile& T, const float*
 {
   ColumnSums c{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
   const float ax = fmaf(W[0], flx, W[2]), ay = fmaf(W[3], flx, W[5]);
-  if (!covered)
+  if (!kWindow || !covered)
+  {
     c = px_column_checked(tar, w, h, T, ref_col, px, py, W[0], W[1], W[2], W[3], W[4], W[5], flx, t0, ry, lat ? 1 : 0);
-  else if (lat)
+    return c;
+  }
+  if (lat)
     c = px_column_lattice(T.s + ((int)(py + fmaf(W[4], (float)-ry, ay)) - T.oy) * T.bx + ((int)(px + ax) - T.ox), T.bx,
                           ref_col, w, t0, ry);
   else
@@ -1693,7 +1697,11 @@ constexpr int icgn_min_blocks(int warps) { return DIC_ICGN_RESIDENT_WARPS / warp
 #endif
 constexpr int icgn_persistent_min_blocks(int warps) { return DIC_ICGN_PERSISTENT_RESIDENT_WARPS / warps; }
 // The pixel-window kernels' resident warps (px_column_rows): 20, 96 registers.
-constexpr int px_min_blocks(int warps) { return 20 / warps; }
+// Without windows (mode 0) every sample goes through the checked loop, which waits on the global
+// plane and wants warps, not registers: the table kernels' numbers (r 15, 63 504 POIs: 20 warps 1.01
+// ms, 32 0.68).
+constexpr int px_min_blocks(int warps, int mode) { return mode == 0 ? icgn_persistent_min_blocks(warps) : 20 / warps; }
+constexpr int pair_px_min_blocks(int warps, int mode) { return mode == 0 ? icgn_min_blocks(warps) : 20 / warps; }
 
 template <bool kColumn, int kWarps = 4>
 __global__ void __launch_bounds__(kWarps * 32, icgn_min_blocks(kWarps)) k_icgn(IcgnParams P)
@@ -1804,6 +1812,7 @@ __device__ __forceinline__ bool pair_class_sums(const IcgnParams& P, int k, int 
 // The same nine sums under pixel sampling (T: the POI's staged window), by px_column.  `covered`:
 // every sample of the subset lies in the interpolation range and has its support in the window
 // (window_covers, once per iteration); `lat`: on the pixel lattice.
+template <bool kWindow>
 __device__ __forceinline__ bool pair_class_sums_px(const IcgnParams& P, const PixelTile& T, int k, int lane, float px,
                                                    float py, int cx, int cy, float t0, const float (&W)[6], bool covered,
                                                    bool lat, float (&s)[9])
@@ -1814,7 +1823,7 @@ __device__ __forceinline__ bool pair_class_sums_px(const IcgnParams& P, const Pi
   const unsigned mask = __ballot_sync(kFull, c < 2 * rx + 1);
   ColumnSums cs{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
   if (c < 2 * rx + 1)
-    cs = px_column(T, P.tar, P.ref_pack + (size_t)(cy - ry) * w + cx + (c - rx), w, P.h, px, py, W, flx, t0, ry, covered,
+    cs = px_column<kWindow>(T, P.tar, P.ref_pack + (size_t)(cy - ry) * w + cx + (c - rx), w, P.h, px, py, W, flx, t0, ry, covered,
                    lat, mask);
   const bool any_bad = __any_sync(kFull, cs.bad != 0);
   s[0] = warp_sum(cs.A0);
@@ -1858,7 +1867,7 @@ struct PairExchange
 // One POI (queue index i) on one warp (kPoiWarps 1) or on the two warps of a pair
 // (kPoiWarps 2: this warp walks class `cls`, barrier `bar` joins the pair).  Same rules,
 // status codes and outputs as icgn_solve; class 0's lane 0 writes the record.
-template <int kPoiWarps, int kSrc = kSrcTable>
+template <int kPoiWarps, int kSrc = kSrcTable, bool kWindow = true>
 __device__ __forceinline__ void icgn_solve_pair(const IcgnParams& P, int64_t i, int lane, int cls,
                                                 PairExchange* xch, int bar, const PixelTile& T = PixelTile{})
 {
@@ -1895,11 +1904,11 @@ __device__ __forceinline__ void icgn_solve_pair(const IcgnParams& P, int64_t i, 
     if constexpr (kSrc == kSrcPixels)
     {
       lat = on_lattice(W, px, py);
-      covered = window_covers(W, px, py, rx, ry, (float)(w - 2), (float)(h - 2), T, lane);
+      covered = kWindow && window_covers(W, px, py, rx, ry, (float)(w - 2), (float)(h - 2), T, lane);
     }
     const auto class_sums = [&](int k, float(&out)[9]) {
       if constexpr (kSrc == kSrcPixels)
-        return pair_class_sums_px(P, T, k, lane, px, py, cx, cy, t0, W, covered, lat, out);
+        return pair_class_sums_px<kWindow>(P, T, k, lane, px, py, cx, cy, t0, W, covered, lat, out);
       else
         return pair_class_sums(P, k, lane, px, py, cx, cy, t0, W, out);
     };
@@ -2317,9 +2326,14 @@ __device__ __forceinline__ bool px_stage(const IcgnParams& P, int64_t i, int lan
                                          PixelTile& T, int cls = 0, int* verdict = nullptr, int pair_bar = 0)
 {
   constexpr int mode = kMode;
+  if constexpr (mode == 0)
+  {
+    T = PixelTile{};
+    return true;
+  }
   const int bx = px_window_x(P.rx), by = px_window_y(P.ry);
   int ox = 0, oy = 0, fits = 0;
-  if (lane == 0 && mode != 0)
+  if (lane == 0)
   {
     fits = px_origin(P, P.pois + i, bx, by, ox, oy);
     if (fits)
@@ -2445,6 +2459,7 @@ __device__ __forceinline__ void icgn_store(dic_poi* poi, const float* ref, const
 
 // One POI (queue index i) on the calling warp under pixel sampling, column walk: icgn_solve's
 // rules, codes and outputs from the staged window T.  ref: the warp's copy of the POI's record.
+template <bool kWindow>
 __device__ __forceinline__ void icgn_solve_px(const IcgnParams& P, int64_t i, int lane, const PixelTile& T,
                                               const float* ref)
 {
@@ -2478,8 +2493,9 @@ __device__ __forceinline__ void icgn_solve_px(const IcgnParams& P, int64_t i, in
   {
     ++it;
     ColumnSums c{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
-    const bool covered = window_covers(W, px, py, rx, ry, xmax, ymax, T, lane);
-    if (col_active) c = px_column(T, P.tar, ref_col, w, h, px, py, W, flx, t0, ry, covered, on_lattice(W, px, py), mask);
+    const bool covered = kWindow && window_covers(W, px, py, rx, ry, xmax, ymax, T, lane);
+    if (col_active)
+      c = px_column<kWindow>(T, P.tar, ref_col, w, h, px, py, W, flx, t0, ry, covered, on_lattice(W, px, py), mask);
     if (__any_sync(kFull, c.bad))
     {
       // Rare path: classify with the CPU's order (src/oc_icgn.cpp:266-301).
@@ -2544,7 +2560,7 @@ __device__ __forceinline__ void ref_store(float* ref, float2 v, int lane)
 // kMode: 2 windows staged by TMA, 1 staged by warp copies, 0 no windows (every sample from
 // the global plane)
 template <int kWarps, int kMode>
-__global__ void __launch_bounds__(kWarps * 32, px_min_blocks(kWarps))
+__global__ void __launch_bounds__(kWarps * 32, px_min_blocks(kWarps, kMode))
     k_icgn_px(IcgnParams P, const __grid_constant__ CUtensorMap map, unsigned long long* next, int* err)
 {
   __shared__ __align__(16) float refs[kWarps][kRefFloats];
@@ -2567,7 +2583,7 @@ __global__ void __launch_bounds__(kWarps * 32, px_min_blocks(kWarps))
     const float2 rv = ref_fetch(P, i, lane);
     if (!px_stage<kMode>(P, i, lane, win_f, win, &map, bar, parity, err, T)) return;
     ref_store(refs[warp], rv, lane);
-    icgn_solve_px(P, i, lane, T, refs[warp]);
+    icgn_solve_px<kMode != 0>(P, i, lane, T, refs[warp]);
     __syncwarp();   // every lane's reads of this window before the next copy overwrites it
   }
 }
@@ -2605,6 +2621,7 @@ __device__ __forceinline__ float reduce_sums_half(const ColumnSums& c, float flx
 
 // The two halves' POIs (live: this half has one, queue index i), icgn_solve_px's rules and
 // outputs.  T, ref: the half's window and record.
+template <bool kWindow>
 __device__ __forceinline__ void icgn_solve_px_half(const IcgnParams& P, int64_t i, bool live, int lane,
                                                    const PixelTile& T, const float* ref)
 {
@@ -2647,10 +2664,10 @@ __device__ __forceinline__ void icgn_solve_px_half(const IcgnParams& P, int64_t 
   while (__any_sync(kFull, run))
   {
     ColumnSums c{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
-    const bool covered = window_covers(W, px, py, rx, ry, xmax, ymax, T, h16, half);
+    const bool covered = kWindow && window_covers(W, px, py, rx, ry, xmax, ymax, T, h16, half);
     const bool lat = on_lattice(W, px, py), col = run && h16 < sw;
     const unsigned rows = __ballot_sync(kFull, col && covered && !lat);
-    if (col) c = px_column<true>(T, P.tar, ref_col, w, h, px, py, W, flx, t0, ry, covered, lat, rows);
+    if (col) c = px_column<kWindow, true>(T, P.tar, ref_col, w, h, px, py, W, flx, t0, ry, covered, lat, rows);
     __syncwarp();
     const unsigned bad = __ballot_sync(kFull, c.bad != 0);
     if (bad)
@@ -2717,10 +2734,15 @@ template <int kMode>
 __device__ __forceinline__ bool px_stage_half(const IcgnParams& P, int64_t i, bool live, int lane, int win_f, uint32_t win,
                                               const CUtensorMap* map, uint32_t bar, uint32_t& parity, int* err, PixelTile& T)
 {
+  if constexpr (kMode == 0)
+  {
+    T = PixelTile{};
+    return true;
+  }
   const int bx = px_window_x(P.rx), by = px_window_y(P.ry);
   const int h16 = lane & (kHalf - 1);
   int ox = 0, oy = 0, fits = 0;
-  if (h16 == 0 && live && kMode != 0)
+  if (h16 == 0 && live)
   {
     fits = px_origin(P, P.pois + i, bx, by, ox, oy);
     if (fits)
@@ -2767,7 +2789,7 @@ __device__ __forceinline__ bool px_stage_half(const IcgnParams& P, int64_t i, bo
 }
 
 template <int kWarps, int kMode>
-__global__ void __launch_bounds__(kWarps * 32, px_min_blocks(kWarps))
+__global__ void __launch_bounds__(kWarps * 32, px_min_blocks(kWarps, kMode))
     k_icgn_px_half(IcgnParams P, const __grid_constant__ CUtensorMap map, unsigned long long* next, int* err)
 {
   __shared__ __align__(16) float refs[2 * kWarps][kRefFloats];
@@ -2796,7 +2818,7 @@ __global__ void __launch_bounds__(kWarps * 32, px_min_blocks(kWarps))
     if (!px_stage_half<kMode>(P, i, live, lane, win_f, win, &map, bar, parity, err, T)) return;
     if (h16 < kRefFloats / 4) reinterpret_cast<float4*>(refs[slot])[h16] = rv;
     __syncwarp();
-    icgn_solve_px_half(P, i, live, lane, T, refs[slot]);
+    icgn_solve_px_half<kMode != 0>(P, i, live, lane, T, refs[slot]);
     __syncwarp();   // both halves' reads of the windows before the next copies overwrite them
   }
 }
@@ -2828,7 +2850,7 @@ __device__ __forceinline__ int64_t pair_fetch(unsigned long long* next, long lon
 // kMode as in k_icgn_px (2 TMA, 1 warp copies, 0 no windows).  Same bits for every kPoiWarps,
 // kWarps and kMode.
 template <int kPoiWarps, int kWarps, int kMode>
-__global__ void __launch_bounds__(kWarps * 32, px_min_blocks(kWarps))
+__global__ void __launch_bounds__(kWarps * 32, pair_px_min_blocks(kWarps, kMode))
     k_icgn_pair_px(IcgnParams P, const __grid_constant__ CUtensorMap map, unsigned long long* next, int* err)
 {
   constexpr int kSlots = kWarps / kPoiWarps;
@@ -2851,7 +2873,7 @@ __global__ void __launch_bounds__(kWarps * 32, px_min_blocks(kWarps))
     PixelTile T;
     if (!px_stage<kMode, kPoiWarps>(P, i, lane, win_f, win, &map, bar, parity, err, T, cls, verdict[slot], 1 + slot))
       return;
-    icgn_solve_pair<kPoiWarps, kSrcPixels>(P, i, lane, cls, &xch[slot], 1 + slot, T);
+    icgn_solve_pair<kPoiWarps, kSrcPixels, kMode != 0>(P, i, lane, cls, &xch[slot], 1 + slot, T);
     __syncwarp();
   }
 }
@@ -2936,7 +2958,7 @@ __device__ __forceinline__ int batch_job_of(const BatchJob* __restrict__ jobs, i
 // kMode 2: every job has a map (TMA windows); 1: warp copies for all.  32 resident warps per
 // SM (64 registers, no spills), as k_icgn_px.
 template <int kWarps, int kMode>
-__global__ void __launch_bounds__(kWarps * 32, px_min_blocks(kWarps))
+__global__ void __launch_bounds__(kWarps * 32, px_min_blocks(kWarps, kMode))
     k_icgn_batch_px(const BatchJob* __restrict__ jobs, int njobs, dic_poi* pois, const PoiRef* poi_ref, int64_t begin,
                     int64_t end, unsigned long long* next, float conv, float max_iter, unsigned long long* iter_sum,
                     uint32_t win_bytes, uint32_t wait_polls, int* err)
@@ -2976,7 +2998,7 @@ __global__ void __launch_bounds__(kWarps * 32, px_min_blocks(kWarps))
     const float2 rv = ref_fetch(P, k, lane);
     if (!px_stage<kMode>(P, k, lane, win_f, win, J.map, bar, parity, err, T)) return;
     ref_store(refs[warp], rv, lane);
-    icgn_solve_px(P, k, lane, T, refs[warp]);
+    icgn_solve_px<true>(P, k, lane, T, refs[warp]);
     __syncwarp();
   }
 }
@@ -3034,7 +3056,7 @@ __global__ void __launch_bounds__(kWarps * 32, icgn_min_blocks(kWarps))
 // k_icgn_pair_px's windows (each job's map in device memory, win_bytes the window of the
 // launch's largest radius).  kMode 2: TMA windows (every job has a map), 0: no windows.
 template <int kPoiWarps, int kWarps, int kMode>
-__global__ void __launch_bounds__(kWarps * 32, px_min_blocks(kWarps))
+__global__ void __launch_bounds__(kWarps * 32, pair_px_min_blocks(kWarps, kMode))
     k_icgn_batch_pair_px(const BatchJob* __restrict__ jobs, int njobs, dic_poi* pois, const PoiRef* poi_ref,
                          int64_t begin, int64_t end, unsigned long long* next, float conv, float max_iter,
                          unsigned long long* iter_sum, uint32_t win_bytes, uint32_t wait_polls, int* err)
@@ -3075,7 +3097,7 @@ __global__ void __launch_bounds__(kWarps * 32, px_min_blocks(kWarps))
     PixelTile T;
     if (!px_stage<kMode, kPoiWarps>(P, k, lane, win_f, win, J.map, bar, parity, err, T, cls, verdict[slot], 1 + slot))
       return;
-    icgn_solve_pair<kPoiWarps, kSrcPixels>(P, k, lane, cls, &xch[slot], 1 + slot, T);
+    icgn_solve_pair<kPoiWarps, kSrcPixels, kMode != 0>(P, k, lane, cls, &xch[slot], 1 + slot, T);
     __syncwarp();
   }
 }
