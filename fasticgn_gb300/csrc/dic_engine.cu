@@ -239,8 +239,9 @@ struct dic_cnn
   X(34, 8, true) X(36, 8, false) X(38, 5, true) X(40, 4, false) X(42, 3, false) X(44, 5, false) X(46, 2, true) \
   X(48, 2, false) X(50, 3, false) X(52, 3, false) X(54, 1, false) X(56, 1, false) X(58, 1, true) X(60, 1, false) \
   X(62, 1, true) X(64, 1, false)
-// CTAs of a second pass, and of a pass behind a device switch, at most: near ties are rare, and
-// so are the frames that switch a repair pass on
+// CTAs of a second pass, and of a pass behind a device switch, at most (eight on each of 152 SMs;
+// they walk what there is): near ties are rare where a window has texture, and so are the frames
+// that switch a repair pass on
 constexpr unsigned kFewCtas = 1216;
 unsigned fftcc_grid(const FftccParams& p, int per_cta)
 {
