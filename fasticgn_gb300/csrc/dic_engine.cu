@@ -252,7 +252,7 @@ template <int M, int kPois, bool kPrime>
 void launch_fftcc_line(const FftccParams& p, cudaStream_t st)
 {
   using F = FftccLine<M, kPois>;
-  k_fftcc_line<M, kPois><<<fftcc_grid(p, kPois), F::kThreads, F::kSmem, st>>>(p);
+  if (p.near) k_fftcc_line<M, kPois><<<fftcc_grid(p, kPois), F::kThreads, F::kSmem, st>>>(p);
   const unsigned second = (unsigned)std::min<int64_t>(p.n, kFewCtas);
   if constexpr (kPrime)
     k_fftcc_large<<<second, 256, (size_t)2 * M * (M + 1) * sizeof(float2), st>>>(p, M);
@@ -263,12 +263,30 @@ template <int M>
 void launch_fftcc2(const FftccParams& p, cudaStream_t st)
 {
   const unsigned blocks = fftcc_grid(p, 4);
-  if (p.enable) k_fftcc2<M, false, true><<<blocks, 64, 0, st>>>(p);
-  else k_fftcc2<M><<<blocks, 64, 0, st>>>(p);
+  if (p.near || !fftcc2_near(M))   // else the plain order alone
+  {
+    if (p.enable) k_fftcc2<M, false, true><<<blocks, 64, 0, st>>>(p);
+    else k_fftcc2<M><<<blocks, 64, 0, st>>>(p);
+  }
   if constexpr (fftcc2_near(M)) k_fftcc2<M, true><<<std::min(blocks, kFewCtas), 64, 0, st>>>(p);
 }
-// whether a length's launch fills a list of near ties (FftccParams::near)
-bool fftcc_near(int m) { return m > 32 || (m >= 8 && m <= 30 && fftcc2_near(m)); }
+// POIs per SM up to which a queue takes the plain order alone, one launch where the faster kernels
+// need three (the list's reset, the first and the second pass).  us, plain against faster: 2r = 14,
+// 64 POIs 10 / 14, 4 864 17 / 18, 7 300 23 / 22; 28, 64 14 / 16, 2 432 17 / 18, 3 600 25 / 21; 40, 64
+// 12 / 18, 608 15 / 18, 1 216 21 / 22, 1 800 31 / 24; 60, 64 16 / 20, 608 24 / 24, 1 216 43 / 39.
+// The direct 11- and 13-point DFTs cost more sooner (44, 256 20 / 22, 608 25 / 22; 52, 256 22 / 24, 608 35 / 25;
+// 26, 4 POIs 20 / 16), and a 2 x prime length above 32 is never better off (its plain order is the
+// direct DFT).
+int64_t fftcc_plain_per_sm(int m)
+{
+  if (m > 32) return m % 4 == 2 && is_prime(m / 2) ? 0 : fftcc2_near(m) ? 2 : 4;
+  return m == 14 ? 32 : m == 26 ? 0 : 16;
+}
+// whether a length's launch for n POIs fills a list of near ties (FftccParams::near)
+bool fftcc_near(int m, int64_t n, int sms)
+{
+  return (m > 32 || (m >= 8 && m <= 30 && fftcc2_near(m))) && n > fftcc_plain_per_sm(m) * sms;
+}
 // the shared-memory opt-in of every k_fftcc_line form on the current device
 void fftcc_attributes()
 {
@@ -1381,12 +1399,18 @@ struct dic_engine
   }
 
   // ---------------------------------------------------------------- solvers
+  int sm_count() const
+  {
+    int sms = 0;
+    DIC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg.device));
+    return sms;
+  }
   // FFTCC launch for an explicit plane pair and (square) radius; p.near / near_n must be set where
-  // fftcc_near(2 r).
+  // fftcc_near(2 r, n).
   void fftcc_launch(FftccParams p, int r, cudaStream_t on = nullptr)
   {
     cudaStream_t st = on ? on : stream;
-    if (fftcc_near(2 * r))
+    if (fftcc_near(2 * r, p.n, sm_count()))
     {
       DIC_CUDA(cudaMemsetAsync(p.near_n, 0, sizeof(unsigned long long), st));
       ++launches;   // the second pass
@@ -1428,7 +1452,7 @@ struct dic_engine
     FftccParams p{ref_f32.ptr, tar_f32.ptr, d_pois, n, w, h};
     p.n_dev = n_dev;
     p.enable = enable;
-    if (fftcc_near(2 * cfg.subset_radius_x))
+    if (fftcc_near(2 * cfg.subset_radius_x, n, sm_count()))
     {
       fft_near.ensure((size_t)n);
       fft_near_n.ensure(1);

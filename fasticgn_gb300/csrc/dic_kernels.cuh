@@ -3419,6 +3419,7 @@ struct FftccParams
   // factor above 5) leave POIs with another value within kNearTie of their peak to a second launch
   // over near[0 .. *near_n), which decides them in the plain order: the peak does not depend on
   // which kernel is the faster one.
+  // Without a list (a short queue) the second pass's kernel takes the whole queue.
   int64_t* near = nullptr;
   unsigned long long* near_n = nullptr;
 };
@@ -3623,8 +3624,8 @@ __host__ __device__ constexpr bool fftcc2_near(int m)
     if (m % d == 0 && is_prime(d)) return true;
   return false;
 }
-// Two POIs on the calling warp: queue indices i0, i0 + 1, or (kSecond) the entries i0, i0 + 1 of
-// P.near, of which `count` exist; zs: the warp's two windows.
+// Two POIs on the calling warp: queue indices i0, i0 + 1, or (kSecond, where P.near is set) the
+// entries i0, i0 + 1 of P.near, of which `count` exist; zs: the warp's two windows.
 template <int M, bool kSecond>
 __device__ __forceinline__ void fftcc2_warp(const FftccParams& P, int64_t i0, int64_t count, float2* zs)
 {
@@ -3633,7 +3634,7 @@ __device__ __forceinline__ void fftcc2_warp(const FftccParams& P, int64_t i0, in
   constexpr bool kNear = fftcc2_near(M) && !kSecond;
   const int lane = threadIdx.x & 31;
   const int w = P.w, h = P.h;
-  const auto index = [&](int q) { return kSecond ? P.near[i0 + q] : i0 + q; };
+  const auto index = [&](int q) { return kSecond && P.near ? P.near[i0 + q] : i0 + q; };
   // per-POI scalars of the two POIs, kept as named registers (the POI loop is not unrolled,
   // which keeps one copy of the forward transforms in the instruction stream)
   bool live0 = false, live1 = false;
@@ -3839,11 +3840,11 @@ __device__ __forceinline__ void fftcc2_warp(const FftccParams& P, int64_t i0, in
     fftcc_store<M>(P.pois + index(q), best_idx, best, q ? uq1 : uq0, q ? vq1 : vq0, nq);
 }
 
-// entries a launch has to go through: the queue, or (kSecond) the list
+// entries a launch has to go through: the queue, or (kSecond) the list, if there is one
 template <bool kSecond>
 __device__ __forceinline__ int64_t fftcc_count(const FftccParams& P)
 {
-  if constexpr (kSecond) return (int64_t)*P.near_n;
+  if (kSecond && P.near) return (int64_t)*P.near_n;
   if (P.enable && *P.enable == 0) return 0;
   return P.n_dev ? *P.n_dev : P.n;
 }
@@ -4258,14 +4259,14 @@ __device__ __forceinline__ void fftcc_big_poi(const FftccParams& P, int64_t i)
   }
 }
 
-// the POIs of P.near, in the plain order
+// the POIs of P.near, or without a list of the queue, in the plain order
 template <int M>
 __global__ void __launch_bounds__(kBigThreads) k_fftcc_big(FftccParams P)
 {
-  const int64_t listed = (int64_t)*P.near_n;
-  for (int64_t k = blockIdx.x; k < listed; k += gridDim.x)
+  const int64_t count = fftcc_count<true>(P);
+  for (int64_t k = blockIdx.x; k < count; k += gridDim.x)
   {
-    fftcc_big_poi<M>(P, P.near[k]);
+    fftcc_big_poi<M>(P, P.near ? P.near[k] : k);
     __syncthreads();
   }
 }
