@@ -3438,7 +3438,13 @@ __device__ __forceinline__ void leave_near_tie(const FftccParams& P, int64_t i) 
 // the first pass answers: no shift, and zncc 0 / 0.  29 000 POIs at r 20, all flat in both images:
 // both passes whole 0.57 ms, the plain order alone 0.32, now 0.13; all flat in the target only
 // 0.57, 0.32 and 0.46 (at half of the POIs 0.38, 0.32 and 0.33, at a fifth 0.27, 0.32 and 0.26).
-__device__ __forceinline__ bool flat_windows(float rn, float tn) { return rn <= 4e-12f * tn || tn <= 4e-12f * rn; }
+// So does a POI whose map's scale, and with it the margin, is beyond the float range: no difference
+// of two such values says anything.
+template <int M>
+__device__ __forceinline__ bool second_pass_decides(float rn, float tn)
+{
+  return rn <= 4e-12f * tn || tn <= 4e-12f * rn || isinf(0.5f * (rn + tn) * (float)(M * M));
+}
 // k v has at most 24 significant bits for every k <= M^2
 template <int M>
 __device__ __forceinline__ bool flat_exact(float v)
@@ -3720,7 +3726,7 @@ __device__ __forceinline__ void fftcc2_warp(const FftccParams& P, int64_t i0, in
     if (q == 0) { rn0 = rnq; tn0 = tnq; }
     else { rn1 = rnq; tn1 = tnq; }
     if constexpr (kNear)
-      if (flat_windows(rnq, tnq))
+      if (second_pass_decides<M>(rnq, tnq))
       {
         bool zero = rnq == 0.f && tnq == 0.f && flat_exact<M>(rmean) && flat_exact<M>(tmean);
         if (zero && lane < M)
@@ -4563,8 +4569,8 @@ __device__ __forceinline__ void fftcc_line_block(const FftccParams& P, int64_t b
       return v;
     });
   norm = poi_sum(norm);   // its barriers also end the column pass
-  const bool flat = on && flat_windows(norm.x, norm.y);
-  if (flat)
+  const bool settled = on && second_pass_decides<M>(norm.x, norm.y);
+  if (settled)
   {
     // s_zero: every value of the windows is its exact mean
     bool zero = norm.x == 0.f && norm.y == 0.f && flat_exact<M>(mean.x) && flat_exact<M>(mean.y);
@@ -4644,11 +4650,11 @@ __device__ __forceinline__ void fftcc_line_block(const FftccParams& P, int64_t b
     if (j == 0) s_top[qb] = top;
   }
   __syncthreads();
-  if (c != 0 || !(on || flat)) return;
-  if (flat ? !s_zero[q] : s_close[q] > 1)
+  if (c != 0 || !(on || settled)) return;
+  if (settled ? !s_zero[q] : s_close[q] > 1)
     leave_near_tie(P, i);
   else
-    fftcc_store<M>(P.pois + i, flat || s_idx[q] == INT_MAX ? 0 : s_idx[q], flat ? 0.f : s_top[q], ui, vi, norm.x * norm.y);
+    fftcc_store<M>(P.pois + i, settled || s_idx[q] == INT_MAX ? 0 : s_idx[q], settled ? 0.f : s_top[q], ui, vi, norm.x * norm.y);
 }
 
 // grid as k_fftcc2's

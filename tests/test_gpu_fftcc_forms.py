@@ -79,3 +79,23 @@ def test_other_lengths_match_the_oracle(dic, oracle_mod, r):
     ref, tar = pr.ref.astype(np.float32), pr.tar.astype(np.float32)
     O.fftcc2d(ref, tar, oq, r)
     check_fftcc(O, ref, tar, r, q[~out], oq[~out])
+
+
+@pytest.mark.parametrize("r", [14, 17, 20, 27, 31, 32])
+def test_maps_beyond_float_range(dic, r):
+    """Pixels so large that the peak, and with it the margin of a near tie, is infinite: still the
+    plain order's peak, in short and in long queues."""
+    m = 2 * r
+    rng = np.random.default_rng(r)
+    h, w = 4 * r + 30, 4 * r + 40
+    # peak of a perfect match: m^4 var, 2.5 times beyond the range; the rest of the map stays within
+    ref = (rng.normal(size=(h, w)) * np.sqrt(2.5 * 3.4e38) / m ** 2).astype(np.float32)
+    tar = np.roll(ref, (1, 2), (0, 1))
+    q0 = dic.grid_queue(w, h, r, 4)[:299]
+    with dic.Engine(r) as e:
+        e.set_ref(ref)
+        e.set_tar(tar)
+        short, long = e.fftcc(q0.copy()), e.fftcc(np.tile(q0, 5100 // len(q0) + 1))[:len(q0)]
+    for f in ("u", "v"):
+        np.testing.assert_array_equal(long[f], short[f])
+    assert ((long["u"] == 2) & (long["v"] == 1)).all()
