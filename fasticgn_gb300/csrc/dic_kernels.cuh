@@ -3859,9 +3859,12 @@ __device__ __forceinline__ int64_t fftcc_count(const FftccParams& P)
 // a device switch that is off (a stream's repair passes, almost always) then costs 6 us where the
 // full grid's empty CTAs took 34 (162 000 POIs).  The loop costs the transforms their schedule
 // (k_fftcc2<30> 0.65 against 0.61 ms at 2048^2), so launches without a switch go without it.
+// CTAs per SM asked of the compiler (0: its own choice).  2r = 22 keeps the 128 registers that it
+// had before the test of the norms: with 151 it loses an eighth of its warps (262 600 POIs 0.52 ->
+// 0.59 ms; capped 0.53).  Caps elsewhere spill (2r = 30 at 7 or 8 CTAs 0.93 against 0.67 ms at 2048^2).
+constexpr int fftcc2_min_blocks(int m, bool walk) { return m == 22 && !walk ? 8 : 0; }
 template <int M, bool kSecond = false, bool kWalk = kSecond>
-// (Register caps for 7 or 8 CTAs per SM spill: 0.93 against 0.67 ms at 2048^2.)
-__global__ void __launch_bounds__(64) k_fftcc2(FftccParams P)
+__global__ void __launch_bounds__(64, fftcc2_min_blocks(M, kWalk)) k_fftcc2(FftccParams P)
 {
   constexpr int kWarps = 2, S = M + 1;
   __shared__ float2 smem[kWarps * 2][M * S];
