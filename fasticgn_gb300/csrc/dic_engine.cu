@@ -232,9 +232,10 @@ struct dic_cnn
   }
 };
 
-// FFTCC lengths above 32 with the POIs per CTA of k_fftcc_line (as many as fill the warps of the
-// CTA's lines, 34 -> 8 POIs on 272 of 288 threads, while two CTAs or more share an SM) and
-// whether near ties go to the line-DFT kernel (2 x prime) or to k_fftcc_big.
+// FFTCC lengths above 32 with the POIs per CTA of k_fftcc_line (up to 52 as many as fill the warps
+// of the CTA's lines while two CTAs or more share an SM, 34 -> 8 POIs on 272 of 288 threads; above
+// that one, whose window alone takes 24-33 KB; other counts were not timed there) and whether near
+// ties go to the line-DFT kernel (2 x prime) or to k_fftcc_big.
 #define DIC_FFTCC_LINES(X)                                                                             \
   X(34, 8, true) X(36, 8, false) X(38, 5, true) X(40, 4, false) X(42, 3, false) X(44, 5, false) X(46, 2, true) \
   X(48, 2, false) X(50, 3, false) X(52, 3, false) X(54, 1, false) X(56, 1, false) X(58, 1, true) X(60, 1, false) \
@@ -727,8 +728,8 @@ struct dic_engine
   // four-plane table); the autotuner still times both forms.  shape[0]: single queues,
   // shape[1]: batches.
   // The pixel pair walk's default (2 warps per CTA, 2 per POI, TMA windows) is its fastest
-  // measured form on the 2048² pair at r 20 and 30 (with the ungrouped row loop 5.84 and 8.05 ms; 4 warps per
-  // CTA 7.15 and 11.8, 8 warps 7.16 and 12.6, one warp per POI 6.9 and 17.1).
+  // measured form: 27 000 to 29 000 POIs at r 17, 20 and 30 0.45, 0.50 and 0.67 ms; 4 warps per CTA 0.49, 0.55
+  // and 0.73, 8 warps 0.51, 0.56 and 0.74, one warp per POI 0.53, 0.56 and 0.96 at best.
   IcgnShape shape[2][kWalks] = {{{4, 8, 0.f}, {4, 8, 0.f}, {4, 8, 0.f}, {4, 0, 0.f, 1}, {2, 0, 0.f, 1, 2}},
                                 {{4, 7, 0.f}, {4, 7, 0.f}, {4, 7, 0.f}, {4, 0, 0.f}, {2, 0, 0.f, 0, 2}}};
   bool tuned[2][kWalks] = {};

@@ -176,7 +176,8 @@ void launch_ref_planes(const T* raw, int w, int h, float scale, float* ref_f32, 
 // of `pitch` floats (a multiple of 4), for the TMA windows when W itself is not a multiple of
 // 4.  A thread takes one column of four rows, so four loads are in flight and any W and any
 // alignment of `raw` will do.  k_prepare_tar without its table went through its 19x19 halo
-// tiles for this: 2048^2 uint16 27 -> 6.6 us, 1024^2 uint8 8.0 -> 2.9.  The grid is linear (row blocks x column blocks), so any H will do as well.
+// tiles for this: 2048^2 uint16 27 -> 6.6 us, 1024^2 uint8 8.0 -> 2.9.  The grid is linear (row
+// blocks x column blocks), so any H will do as well.
 // --------------------------------------------------------------------------------------
 constexpr int kPlaneThreads = 128, kPlaneRows = 4;
 template <typename T>
@@ -1300,8 +1301,8 @@ __device__ __forceinline__ unsigned px_base()
 // samples come first, and where a lane's support steps otherwise in one of them (its warped
 // column or row crosses a pixel boundary) the warp loads all sixteen pixels of the group's
 // samples (kPerRow: the other twelve of the rows where one does; with two POIs in a warp whole
-// groups without a crossing are rarer).  A subset has an odd number of rows, so the last group has three or one.  `mask`: the
-// calling lanes.
+// groups without a crossing are rarer).  A subset has an odd number of rows, so the last group has
+// three or one.  `mask`: the calling lanes.
 //
 // What bounds it: issue slots (98 instructions a row when every row loaded sixteen pixels, of
 // which 24 are the weights' twelve packed products, two slots of the FMA pipe each) and the
@@ -1309,8 +1310,9 @@ __device__ __forceinline__ unsigned px_base()
 // registers hold a group in flight: 20 resident warps do better than the 32 that 64 registers
 // allowed.  IC-GN on a 2048x2048 pair, 254 016 POIs, r 15: 3.18 -> 2.75 ms with the lattice loop
 // below (with a test per row instead of one per group 2.86, with the texels loaded first 2.79;
-// 16 warps 2.90, 24 warps 2.87); r 30, 36 864 POIs 1.31 -> 1.00 (28 warps 1.11); r 7, two POIs a
-// warp, 171 024 POIs: 0.71 with a test per row, 0.73 per group.  Scalar weights and packed sums moved the time by 1 % or less either way.
+// 16 warps 2.90, 24 warps 2.87); r 30, 36 864 POIs 1.31 -> 1.00 (28 warps 1.11); with two POIs a
+// warp (k_icgn_px_half) a test per group is 3 % slower than one per row.  Scalar weights and packed
+// sums moved the time by 1 % or less either way.
 struct ColumnRows
 {
   float q[4][4];
@@ -1696,9 +1698,10 @@ constexpr int icgn_min_blocks(int warps) { return DIC_ICGN_RESIDENT_WARPS / warp
 #define DIC_ICGN_PERSISTENT_RESIDENT_WARPS 32
 #endif
 constexpr int icgn_persistent_min_blocks(int warps) { return DIC_ICGN_PERSISTENT_RESIDENT_WARPS / warps; }
-// The pixel-window kernels' resident warps (px_column_rows): 20, 96 registers.
+// The pixel-window kernels' resident warps (px_column_rows): 20 at 96 registers, 16 at 128 where a
+// CTA has 8 warps.
 // Without windows (mode 0) every sample goes through the checked loop, which waits on the global
-// plane and wants warps, not registers: the table kernels' numbers (r 15, 63 504 POIs: 20 warps 1.01
+// plane and wants warps, not registers: the table kernels' numbers (r 15, 61 504 POIs: 20 warps 1.01
 // ms, 32 0.68).
 constexpr int px_min_blocks(int warps, int mode) { return mode == 0 ? icgn_persistent_min_blocks(warps) : 20 / warps; }
 constexpr int pair_px_min_blocks(int warps, int mode) { return mode == 0 ? icgn_min_blocks(warps) : 20 / warps; }
@@ -2595,7 +2598,7 @@ __global__ void __launch_bounds__(kWarps * 32, px_min_blocks(kWarps, kMode))
 // that converges first waits for the other (neighbours on the grid rarely differ by more than
 // an iteration).  A half's butterfly over 16 lanes pairs lanes as the 32-lane one does once it
 // has added the idle half's zeros: the same bits as icgn_solve_px.  171 024 POIs at radius 7
-// (1036x186, step 1): IC-GN 1.23 -> 0.69 ms.
+// (1036x186, step 1): IC-GN 1.23 -> 0.72 ms.  Bound by issue (72 % of slots at 20 warps).
 // --------------------------------------------------------------------------------------
 constexpr int kHalf = 16;
 // reduce_sums over the calling half (h: lane in it): the value v of {B0..B5, A1, A2} is left on
@@ -2955,8 +2958,8 @@ __device__ __forceinline__ int batch_job_of(const BatchJob* __restrict__ jobs, i
 // TMA copies as in k_icgn_px; a job without one (row pitch not a multiple of 16 bytes) is
 // staged by warp copies.  win_bytes is the window slot of the largest radius in the launch.
 // Same bits as each job's single-pair pixel solve.  The copy wait is bounded as in k_icgn_px.
-// kMode 2: every job has a map (TMA windows); 1: warp copies for all.  32 resident warps per
-// SM (64 registers, no spills), as k_icgn_px.
+// kMode 2: every job has a map (TMA windows); 1: warp copies for all.  Resident warps as
+// k_icgn_px's (px_min_blocks).
 template <int kWarps, int kMode>
 __global__ void __launch_bounds__(kWarps * 32, px_min_blocks(kWarps, kMode))
     k_icgn_batch_px(const BatchJob* __restrict__ jobs, int njobs, dic_poi* pois, const PoiRef* poi_ref, int64_t begin,
@@ -4076,8 +4079,9 @@ __global__ void __launch_bounds__(256) k_fftcc_large(FftccParams P, int m)
 }
 
 // --------------------------------------------------------------------------------------
-// The second pass of 32 < M <= 64 where M is not 2 x prime: the near ties that k_fftcc_line lists,
-// in this kernel's own order of operations.  One 128-thread CTA per POI, the packed window z = ref + i tar in shared memory ([M][M + 1] float2; consecutive lanes
+// 32 < M <= 64 where M is not 2 x prime, in the plain order: the near ties that k_fftcc_line lists
+// (the second pass), and short queues whole.  One 128-thread CTA per POI, the packed window
+// z = ref + i tar in shared memory ([M][M + 1] float2; consecutive lanes
 // take consecutive lines, whose odd float2 stride keeps a warp's accesses conflict-free in
 // both directions), every line transform a four-step FFT M = N1 * N2 done in place by
 // small register FFTs:
@@ -4297,12 +4301,14 @@ __global__ void __launch_bounds__(kBigThreads) k_fftcc_big(FftccParams P)
 // imaginary parts (as in k_fftcc2).  Argmax with the CPU's tie rule: the POI's maximum first, its
 // lowest index from the rows that hold it.
 //
-// Bound by instruction issue.  k_fftcc_big (128 threads a POI, lines split over threads, a runtime
-// index and a table twiddle per element, all lines on the way back) issues 2.5 times the
-// instructions; lengths 2 x prime ran as direct DFTs (k_fftcc_large).  Both remain for near ties.
-// Before and now: r 20, 29 000 POIs 0.315 -> 0.208 ms; r 30, 36 864 POIs 0.89 -> 0.70 ms; r 31,
-// 9 396 POIs 1.85 -> 0.39 ms; r 17, 30 000 POIs 2.18 -> 0.25 ms.  (k_fftcc2<14> with the paired
-// 7-point DFT, 171 024 POIs: 0.32 -> 0.20 ms.)
+// At 2r = 60 the waits at the CTA's barriers lead (2.0 cycles an issue), then instruction fetch
+// (1.2: a line's code is long and straight); shared-memory pipe 54 %, issue slots 40 % busy at 167
+// registers.  k_fftcc_big (128 threads a POI, lines split over threads, a runtime index and a table
+// twiddle per element, all lines on the way back) was bound by issue; lengths 2 x prime ran as
+// direct DFTs (k_fftcc_large).  Both remain for near ties, k_fftcc_big for short queues too.
+// Before and now: r 20, 29 000 POIs 0.317 -> 0.206 ms; r 30, 36 864 POIs 0.89 -> 0.66; r 31, 9 396
+// POIs 1.84 -> 0.32; r 17, 28 908 POIs 2.12 -> 0.22.  (k_fftcc2<14> with the paired 7-point DFT,
+// 171 024 POIs: 0.32 -> 0.20 ms.)
 // --------------------------------------------------------------------------------------
 __host__ __device__ constexpr int gcd(int a, int b) { return b ? gcd(b, a % b) : a; }
 __host__ __device__ constexpr int line_n1(int m)

@@ -291,7 +291,8 @@ typedef struct dic_launch_shape
 {
   int32_t warps_per_cta;
   int32_t ctas_per_sm;   /* > 0: persistent launch with this many resident CTAs per SM drawing POIs
-                            from an atomic counter; 0: one CTA per warps_per_cta POIs */
+                            from an atomic counter; 0: one CTA per warps_per_cta POIs (pixel
+                            sampling, walks 3 and 4: persistent at full occupancy) */
   int32_t tuned;
   float ms;              /* best candidate's time, when tuned */
   int32_t tile;          /* column-walk IC-GN only: 0 gathers texels from the coefficient table;
