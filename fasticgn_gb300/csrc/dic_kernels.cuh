@@ -1704,6 +1704,8 @@ constexpr int icgn_persistent_min_blocks(int warps) { return DIC_ICGN_PERSISTENT
 // plane and wants warps, not registers: the table kernels' numbers (r 15, 61 504 POIs: 20 warps 1.01
 // ms, 32 0.68).
 constexpr int px_min_blocks(int warps, int mode) { return mode == 0 ? icgn_persistent_min_blocks(warps) : 20 / warps; }
+// The pair walk at 16, 20, 24 and 28 warps, 27 000 to 29 000 POIs: r 16 0.458, 0.430, 0.428, 0.439
+// ms; r 20 0.535, 0.501, 0.503, 0.522; r 26 0.637, 0.601, 0.606, 0.634; r 31 0.723, 0.677, 0.692, 0.782.
 constexpr int pair_px_min_blocks(int warps, int mode) { return mode == 0 ? icgn_min_blocks(warps) : 20 / warps; }
 
 template <bool kColumn, int kWarps = 4>
