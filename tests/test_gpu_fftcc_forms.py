@@ -99,3 +99,32 @@ def test_maps_beyond_float_range(dic, r):
     for f in ("u", "v"):
         np.testing.assert_array_equal(long[f], short[f])
     assert ((long["u"] == 2) & (long["v"] == 1)).all()
+
+
+@pytest.mark.parametrize("r", [20, 24, 28, 30, 32])
+def test_zncc_error_is_the_plain_orders(dic, r):
+    """Rms distance of zncc from 64 bits: the long queue's form within 5 % of the plain order's."""
+    rng = np.random.default_rng(5)
+    h, w = 260, 420
+    ref = rng.normal(size=(h, w))
+    for _ in range(3):
+        ref = (ref + np.roll(ref, 1, 0) + np.roll(ref, 1, 1)) / 3
+    ref = 128 + 50 * ref / ref.std()
+    a, b = (np.clip(np.rint(im + rng.normal(0, 2, (h, w))), 0, 255).astype(np.uint8)
+            for im in (ref, np.roll(ref, (1, 2), (0, 1))))
+    q0 = dic.grid_queue(w, h, r, 4)
+    q0 = np.ascontiguousarray(q0[:: max(1, len(q0) // 1500)])
+    with dic.Engine(r) as e:
+        e.set_ref(a)
+        e.set_tar(b)
+        plain = np.concatenate([e.fftcc(q0[k:k + 299].copy()) for k in range(0, len(q0), 299)])
+        long = e.fftcc(np.tile(q0, 2000 // len(q0) + 1))[:len(q0)]
+    exact = []
+    for p in q0:
+        x, y = int(p["x"]), int(p["y"])
+        f, g = (im[y - r:y + r, x - r:x + r].astype(np.float64) for im in (a, b))
+        f, g = f - f.mean(), g - g.mean()
+        c = np.fft.irfft2(np.conj(np.fft.rfft2(f)) * np.fft.rfft2(g), s=f.shape)
+        exact.append(c.max() / np.sqrt((f * f).sum() * (g * g).sum()))
+    rms = [float(np.sqrt(np.mean((q["zncc"] - np.array(exact)) ** 2))) for q in (plain, long)]
+    assert rms[1] <= 1.05 * rms[0], rms
