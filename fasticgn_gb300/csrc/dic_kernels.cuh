@@ -4671,9 +4671,12 @@ __device__ __forceinline__ void fftcc_line_block(const FftccParams& P, int64_t b
     fftcc_store<M>(P.pois + i, settled || s_idx[q] == INT_MAX ? 0 : s_idx[q], settled ? 0.f : s_top[q], ui, vi, norm.x * norm.y);
 }
 
-// grid as k_fftcc2's
+// grid as k_fftcc2's.  CTAs per SM asked of the compiler (0: its own choice) where the test of the
+// norms had taken it to the next step of registers: 2r = 38, 45 018 POIs 0.43 -> 0.40 ms; 56, 42 898
+// 0.85 -> 0.75.
+constexpr int fftcc_line_min_blocks(int m) { return m == 38 ? 4 : m == 56 ? 5 : 0; }
 template <int M, int kPois>
-__global__ void __launch_bounds__(FftccLine<M, kPois>::kThreads) k_fftcc_line(FftccParams P)
+__global__ void __launch_bounds__(FftccLine<M, kPois>::kThreads, fftcc_line_min_blocks(M)) k_fftcc_line(FftccParams P)
 {
   const int64_t count = fftcc_count<false>(P);
   for (int64_t base = (int64_t)blockIdx.x * kPois; base < count; base += (int64_t)gridDim.x * kPois)
