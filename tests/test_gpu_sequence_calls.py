@@ -7,15 +7,16 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("radius", [7, 10, 20])     # with and without the FFTCC's list of near ties
-def test_calls_between_frames(dic, radius):
+# the FFTCC in the plain order (7; 20 with 396 POIs), without near ties (10) and with their list
+@pytest.mark.parametrize("radius,step", [(7, 6), (10, 6), (20, 6), (20, 9)])
+def test_calls_between_frames(dic, radius, step):
     from fasticgn_gb300 import speckle
     pr = speckle.pair_bumps(seed=radius, width=240, height=200, max_disp=2.0, max_strain=0.01)
     ref = pr.ref.copy()
     ref[:, :80] = np.tile(np.random.default_rng(3).integers(0, 255, (2, 2)), (100, 40))   # every shift ties
     jump = np.roll(ref, (radius // 2, radius - 2), (0, 1))             # the whole frame is solved again
     frames = [pr.tar, ref, pr.tar, jump, pr.tar.astype(np.float32), jump.astype(np.float32)]
-    tmpl = dic.grid_queue(240, 200, radius, 6)
+    tmpl = dic.grid_queue(240, 200, radius, step)
     more = dic.grid_queue(240, 200, radius, 2)
     runs = []
     for graphs in (True, False):
